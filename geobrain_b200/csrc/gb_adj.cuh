@@ -267,7 +267,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                     const int gz = z0 + rv;
                     if (fast || (gz < g.Nz && gx0 < g.Nx)) {
                         float Dx[4], Dz[4];
-                        float4 mp1;
+                        const float4 mp1 = wp[u + R - 1];       // mu_p row rr
                         grad_x4<R>(sP + rr * RW, lane, g.c, Dx, mp1);
                         grad_z4<R>(wp, u, g.c, Dz);
                         const float4 vx1 = lds4(sVX + rr * VXW + 4 * lane + 4);
@@ -396,7 +396,10 @@ constexpr size_t adj_smem_bytes()
 //   G1 = sum(mu_p1 * I), G2 = sum(mu_v1 * J) over groups (compensated),
 //   dL/dc = 2 G1 / c, dL/dden = (G1 + G2) / den,
 // then the adjoint of pad_model: each model cell collects every padded cell
-// it was replicated into (acoustic_2d.py:55-64).  Internal linkage: the
+// it was replicated into (acoustic_2d.py:55-64).  An interior cell was copied
+// nowhere; one on the model's edge collects a strip of the frame and a corner
+// cell nabc^2 cells of it, times the groups: a warp shares those (one thread
+// per corner took 0.2 to 0.7 ms, most of the kernel's time).  Internal linkage: the
 // translation units that instantiate the step kernels include this header too.
 static __global__ void grad_finish_kernel(const float *__restrict__ vp, const float *__restrict__ rho,
                                    const float *__restrict__ G1, const float *__restrict__ C1,
@@ -404,31 +407,67 @@ static __global__ void grad_finish_kernel(const float *__restrict__ vp, const fl
                                    long long plane, int nz, int nx, int pml, int pitch, float *grad_vp,
                                    float *grad_rho)
 {
+    auto write = [&](long long idx, float g1, float g2) {
+        const float c = vp[idx], den = rho[idx];
+        grad_vp[idx] = 2.f * g1 / c;
+        if (grad_rho) grad_rho[idx] = (g1 + g2) / den;
+    };
+    const int lane = threadIdx.x & 31;
+    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+    // the rim: first and last row, then first and last column without them
+    const long long rows = nz > 1 ? 2LL * nx : nx, cols = nz > 2 ? (nx > 1 ? 2LL : 1LL) * (nz - 2) : 0;
+    for (long long k = warp; k < rows + cols; k += warps) {
+        int iz, ix;
+        if (k < rows) {
+            iz = k < nx ? 0 : nz - 1;
+            ix = (int)(k % nx);
+        } else {
+            iz = 1 + (int)((k - rows) % (nz - 2));
+            ix = k - rows < nz - 2 ? 0 : nx - 1;
+        }
+        // padded rows / columns replicated from this cell
+        const int r0 = iz == 0 ? 0 : iz + pml, r1 = iz == nz - 1 ? nz + 2 * pml - 1 : iz + pml;
+        const int q0 = ix == 0 ? 0 : ix + pml, q1 = ix == nx - 1 ? nx + 2 * pml - 1 : ix + pml;
+        const int nr = r1 - r0 + 1, nq = q1 - q0 + 1;
+        float s1 = 0.f, e1 = 0.f, s2 = 0.f, e2 = 0.f;
+        for (long long m = lane; m < (long long)nr * nq * n_groups; m += 32) {
+            const int j = (int)(m % nq), i = (int)(m / nq % nr), gi = (int)(m / nq / nr);
+            const long long og = gi * plane + (long long)(r0 + i) * pitch + q0 + j;
+            neumaier_add(s1, e1, G1[og]);
+            neumaier_add(s1, e1, C1[og]);
+            if (G2) {
+                neumaier_add(s2, e2, G2[og]);
+                neumaier_add(s2, e2, C2[og]);
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const float t1 = __shfl_down_sync(0xffffffffu, s1, o), u1 = __shfl_down_sync(0xffffffffu, e1, o);
+            const float t2 = __shfl_down_sync(0xffffffffu, s2, o), u2 = __shfl_down_sync(0xffffffffu, e2, o);
+            neumaier_add(s1, e1, t1);
+            neumaier_add(s2, e2, t2);
+            e1 += u1;
+            e2 += u2;
+        }
+        if (lane == 0) write((long long)iz * nx + ix, s1 + e1, s2 + e2);
+    }
     const long long n = (long long)nz * nx;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < n;
          idx += (long long)gridDim.x * blockDim.x) {
         const int iz = (int)(idx / nx), ix = (int)(idx % nx);
-        const float c = vp[idx], den = rho[idx];
-        // padded rows / columns replicated from this cell
-        const int r0 = iz == 0 ? 0 : iz + pml, r1 = iz == nz - 1 ? nz + 2 * pml - 1 : iz + pml;
-        const int q0 = ix == 0 ? 0 : ix + pml, q1 = ix == nx - 1 ? nx + 2 * pml - 1 : ix + pml;
+        if (iz == 0 || iz == nz - 1 || ix == 0 || ix == nx - 1) continue;
+        const long long o = (long long)(iz + pml) * pitch + ix + pml;
         float s1 = 0.f, e1 = 0.f, s2 = 0.f, e2 = 0.f;
-        for (int i = r0; i <= r1; ++i)
-            for (int j = q0; j <= q1; ++j) {
-                const long long o = (long long)i * pitch + j;
-                for (int gi = 0; gi < n_groups; ++gi) {
-                    const long long og = gi * plane + o;
-                    neumaier_add(s1, e1, G1[og]);
-                    neumaier_add(s1, e1, C1[og]);
-                    if (G2) {
-                        neumaier_add(s2, e2, G2[og]);
-                        neumaier_add(s2, e2, C2[og]);
-                    }
-                }
+        for (int gi = 0; gi < n_groups; ++gi) {
+            const long long og = gi * plane + o;
+            neumaier_add(s1, e1, G1[og]);
+            neumaier_add(s1, e1, C1[og]);
+            if (G2) {
+                neumaier_add(s2, e2, G2[og]);
+                neumaier_add(s2, e2, C2[og]);
             }
-        const float g1 = s1 + e1, g2 = s2 + e2;
-        grad_vp[idx] = 2.f * g1 / c;
-        if (grad_rho) grad_rho[idx] = (g1 + g2) / den;
+        }
+        write(idx, s1 + e1, s2 + e2);
     }
 }
 

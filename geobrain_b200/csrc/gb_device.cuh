@@ -109,6 +109,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
 // completes.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, uint32_t max_polls = kMaxPolls)
 {
+#pragma unroll 1   // unrolled, this is about 190 instructions at each of its uses
     for (uint32_t i = 0; i < max_polls; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if (i > 64) __nanosleep(256);
@@ -149,8 +150,12 @@ __device__ __forceinline__ float at(const float4 &v, int q)
 //   kImgF32   fp32;
 //   kImgBF16  bf16, the upper 16 bits of the fp32 rounded to nearest even;
 //   kImgF24   the upper 24 bits of the fp32 (sign, 8-bit exponent, 15-bit
-//             mantissa) rounded to nearest even, 3 bytes, packed 4 values to
-//             3 words.
+//             mantissa) rounded to nearest even, 3 bytes; per 32 values the
+//             32 upper halves (64 bytes), then the 32 low bytes, so that a
+//             warp's quads are whole sectors of both (as 3 packed words per
+//             quad, each of a quad's stores and loads touched every sector
+//             of the row: the forward step that keeps them took 16 us longer
+//             than one that does not, at 32 shots of 400 x 1200).
 // Both short formats keep the fp32 exponent, so no scale is needed and
 // widening back is exact.  `o` is an element offset, a multiple of 4.
 constexpr int kImgF32 = 0;
@@ -163,12 +168,18 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
-// fp32 -> upper 24 bits, round to nearest even on the 8 dropped bits (a carry
-// into the exponent is the correct rounding up to the next binade).
+// fp32 rounded to its upper 24 bits, to nearest even on the 8 low bits (a
+// carry into the exponent is the correct rounding up to the next binade); the
+// low 8 bits of the result are not cleared.
 __device__ __forceinline__ uint32_t round24(float x)
 {
     const uint32_t u = __float_as_uint(x);
-    return (u + 0x7fu + ((u >> 8) & 1u)) >> 8;
+    return u + 0x7fu + ((u >> 8) & 1u);
+}
+// the 96-byte block of element o
+__device__ __forceinline__ char *block24(const float *base, long long o)
+{
+    return const_cast<char *>(reinterpret_cast<const char *>(base)) + 96 * (o >> 5);
 }
 __device__ __forceinline__ void store_img4(float *base, long long o, int fmt, float4 v)
 {
@@ -177,16 +188,17 @@ __device__ __forceinline__ void store_img4(float *base, long long o, int fmt, fl
         *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(base) + o) = u;
     } else if (fmt == kImgF24) {
         const uint32_t t0 = round24(v.x), t1 = round24(v.y), t2 = round24(v.z), t3 = round24(v.w);
-        uint32_t *w = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(base) + 3 * o);
-        w[0] = t0 | (t1 << 24);
-        w[1] = (t1 >> 8) | (t2 << 16);
-        w[2] = (t2 >> 16) | (t3 << 8);
+        char *blk = block24(base, o);
+        const int i = (int)(o & 31);
+        *reinterpret_cast<uint2 *>(blk + 2 * i) = make_uint2(__byte_perm(t0, t1, 0x7632), __byte_perm(t2, t3, 0x7632));
+        *reinterpret_cast<uint32_t *>(blk + 64 + i) =
+            __byte_perm(__byte_perm(t0, t1, 0x0051), __byte_perm(t2, t3, 0x5100), 0x7610);
     } else {
         stg4(base + o, v);
     }
 }
-// Imaging values as loaded: 4 fp32 words, 2 bf16x2 words or 3 packed fp24
-// words.  Loading and widening are separate so that the loads can be issued
+// Imaging values as loaded: 4 fp32 words, 2 bf16x2 words, or 2 words of upper
+// halves and one of low bytes (fp24).  Loading and widening are separate so that the loads can be issued
 // well ahead of the use without the widening waiting on them.
 struct ImgRaw {
     uint32_t w0, w1, w2, w3;
@@ -199,8 +211,10 @@ __device__ __forceinline__ ImgRaw load_img_raw(const float *base, long long o, i
         return ImgRaw{u.x, u.y, 0u, 0u};
     }
     if (fmt == kImgF24) {
-        const uint32_t *w = reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(base) + 3 * o);
-        return ImgRaw{__ldg(w), __ldg(w + 1), __ldg(w + 2), 0u};
+        const char *blk = block24(base, o);
+        const int i = (int)(o & 31);
+        const uint2 u = __ldg(reinterpret_cast<const uint2 *>(blk + 2 * i));
+        return ImgRaw{u.x, u.y, __ldg(reinterpret_cast<const uint32_t *>(blk + 64 + i)), 0u};
     }
     const uint4 u = __ldg(reinterpret_cast<const uint4 *>(base + o));
     return ImgRaw{u.x, u.y, u.z, u.w};
@@ -212,8 +226,10 @@ __device__ __forceinline__ float4 decode_img4(const ImgRaw &r, int fmt)
         return make_float4(__uint_as_float(r.w0 << 16), __uint_as_float(r.w0 & 0xffff0000u),
                            __uint_as_float(r.w1 << 16), __uint_as_float(r.w1 & 0xffff0000u));
     if (fmt == kImgF24)
-        return make_float4(__uint_as_float(r.w0 << 8), __uint_as_float(((r.w0 >> 24) | (r.w1 << 8)) << 8),
-                           __uint_as_float(((r.w1 >> 16) | (r.w2 << 16)) << 8), __uint_as_float(r.w2 & 0xffffff00u));
+        return make_float4(__uint_as_float(__byte_perm(r.w0, r.w2, 0x1044) & 0xffffff00u),
+                           __uint_as_float(__byte_perm(r.w0, r.w2, 0x3255) & 0xffffff00u),
+                           __uint_as_float(__byte_perm(r.w1, r.w2, 0x1066) & 0xffffff00u),
+                           __uint_as_float(__byte_perm(r.w1, r.w2, 0x3277) & 0xffffff00u));
     return make_float4(__uint_as_float(r.w0), __uint_as_float(r.w1), __uint_as_float(r.w2), __uint_as_float(r.w3));
 }
 

@@ -313,7 +313,7 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                     const int gz = z0 + rv;
                     if (fast || (gz < g.Nz && gx0 < g.Nx)) {
                         float Dx[4], Dz[4];
-                        float4 pv;
+                        const float4 pv = wp[u + R - 1];        // p row rr
                         grad_x4<R>(sP + rr * RW, lane, g.c, Dx, pv);
                         grad_z4<R>(wp, u, g.c, Dz);
                         float4 vx = lds4(sVX + rr * VXW + 4 * lane + 4);
@@ -390,15 +390,14 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                             sts4(sVX + rr * VXW + 4 * lane + 4, vx);
                             sts4(sVZ + (rv + 2 * R) * RW + 4 * lane, vz);
                         }
-                        if (ENERGY && gz >= g.pml && gz < g.pml + g.nz) {
+                        if (ENERGY) {
+                            // cells off the interior are summed too: the maps'
+                            // readers take the interior only
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
-                                const int gx = gx0 + q;
-                                if (gx >= g.pml && gx < g.pml + g.nx) {
-                                    at(e_p[u], q) = __fmaf_rn(at(pv, q), at(pv, q), at(e_p[u], q));
-                                    at(e_vx[u], q) = __fmaf_rn(at(vx, q), at(vx, q), at(e_vx[u], q));
-                                    at(e_vz[u], q) = __fmaf_rn(at(vz, q), at(vz, q), at(e_vz[u], q));
-                                }
+                                at(e_p[u], q) = __fmaf_rn(at(pv, q), at(pv, q), at(e_p[u], q));
+                                at(e_vx[u], q) = __fmaf_rn(at(vx, q), at(vx, q), at(e_vx[u], q));
+                                at(e_vz[u], q) = __fmaf_rn(at(vz, q), at(vz, q), at(e_vz[u], q));
                             }
                         }
                     }

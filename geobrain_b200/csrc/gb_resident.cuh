@@ -240,7 +240,7 @@ __device__ __forceinline__ void res_v_cells(const ResArgs &A, const ResCtx &C, i
 {
     const StepGeom &g = A.g;
     float Dx[4], Dz[4];
-    float4 pv;
+    const float4 &pv = wp[u + R - 1];     // p row r
     grad_x4<R>(C.sP + r * RS, l, g.c, Dx, pv);
     grad_z4<R>(wp, u, g.c, Dz);
     vx = lds4(C.sVX + r * RS + 4 * l);

@@ -69,19 +69,18 @@ __device__ __forceinline__ void divergence4_split(const float *vxr, int lane, co
 // x-derivative of p at the staggered vx points of 4 adjacent cells:
 //   D[q] = sum_k c_k (p[j+1+k] - p[j-k])        (acoustic_2d.py:248-252)
 // pr: the row of the p rectangle (128 wide, column 0 = x0 - 4); the lane's
-// first column j sits at pr[4*lane].
+// first column j sits at pr[4*lane] and its own cells are f1 (the callers'
+// z-windows hold them).
 template <int R>
-__device__ __forceinline__ void grad_x4(const float *pr, int lane, const float (&c)[4], float (&D)[4], float4 &mid)
+__device__ __forceinline__ void grad_x4(const float *pr, int lane, const float (&c)[4], float (&D)[4], const float4 &f1)
 {
     float f[12];
     {
         const float4 f0 = lds4(pr + 4 * lane - 4);
-        const float4 f1 = lds4(pr + 4 * lane);
         const float4 f2 = lds4(pr + 4 * lane + 4);
         f[0] = f0.x; f[1] = f0.y; f[2] = f0.z; f[3] = f0.w;
         f[4] = f1.x; f[5] = f1.y; f[6] = f1.z; f[7] = f1.w;
         f[8] = f2.x; f[9] = f2.y; f[10] = f2.z; f[11] = f2.w;
-        mid = f1;
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {

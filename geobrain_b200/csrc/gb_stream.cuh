@@ -241,7 +241,7 @@ fwd_stream_kernel(const __grid_constant__ CUtensorMap mP, const __grid_constant_
                 if (gz >= g.Nz || gz >= ze) continue;
                 const int pr = ring_row(gz, base_p), vr = ring_row(gz, base_vz);
                 float Dx[4], Dz[4];
-                float4 pv;
+                const float4 pv = wp[u + R - 1];               // p row gz
                 grad_x4<R>(sP + pr * RW, lane, g.c, Dx, pv);
                 grad_z4<R>(wp, u, g.c, Dz);
                 float4 vx = lds4(sVX + pr * VXW + 4 * lane + 4);
