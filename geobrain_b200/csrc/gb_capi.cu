@@ -172,22 +172,35 @@ struct gb_plan {
         return std::max(2, (tiles_z + n_seg - 1) / n_seg);
     }
     cudaStream_t cap_stream = nullptr;                         // capture origin (never the legacy stream)
-    cudaGraphExec_t gexec = nullptr;
-    std::vector<uintptr_t> gkey;                               // what the instantiated graph baked in
-    // CUDA graphs of chunks of gradient steps (each with what it baked in):
-    // the forward steps that keep their imaging fields, the adjoint steps
-    // over them, and the batched forward / adjoint steps (on a batch's first plan)
+    // CUDA graphs of chunks of steps: the plain forward, the forward steps
+    // that keep their imaging fields, the adjoint steps over them, and the
+    // batched forward / adjoint steps (on a batch's first plan).  `key` is
+    // what a graph's shape depends on (device, kernel, steps, streams), `args`
+    // what its kernels' arguments were made of: with other arguments (another
+    // workspace, other traces) its nodes get new parameters, in order, in
+    // place of a new capture (which took 12 ms of host time for 64 launches
+    // and waited for the device).
     struct GraphSlot {
+        cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
-        std::vector<uintptr_t> key;
+        std::vector<uintptr_t> key, args;
+        std::vector<cudaGraphNode_t> nodes;                    // kernel nodes in launch order
         void release()
         {
             if (exec) cudaGraphExecDestroy(exec);
+            if (graph) cudaGraphDestroy(graph);
             exec = nullptr;
+            graph = nullptr;
             key.clear();
+            args.clear();
+            nodes.clear();
         }
     };
-    GraphSlot g_fwd_img, g_adj, g_batch_fwd, g_batch_adj;
+    // set while a chunk is captured (launches record their nodes) or its
+    // graph's parameters are replaced (launches set them, nothing runs)
+    GraphSlot *recording = nullptr, *updating = nullptr;
+    size_t next_node = 0;
+    GraphSlot g_fwd, g_fwd_img, g_adj, g_batch_fwd, g_batch_adj;
     long long api_launches = 0;                                // host launch calls (kernels and graph replays)
 
     ~gb_plan()
@@ -198,9 +211,7 @@ struct gb_plan {
     }
     void release_graph()
     {
-        if (gexec) cudaGraphExecDestroy(gexec);
-        gexec = nullptr;
-        gkey.clear();
+        g_fwd.release();
         g_fwd_img.release();
         g_adj.release();
         g_batch_fwd.release();
@@ -564,25 +575,55 @@ int launch_tile_flags(gb_plan *P, const StepGeom &g, const float *k1, const floa
     return GB_OK;
 }
 
-// One step kernel launch for shot groups [grp0, grp0 + grp_count).
-// A step kernel launch that may overlap the previous kernel of its stream
-// (programmatic dependent launch): the step kernels wait for it on the device
+// One kernel launch of a step loop, and the one place where such a launch
+// is recorded in, or becomes new parameters of, a graph node (capture_chunk).
+// pdl: it may overlap the previous kernel of its stream (programmatic
+// dependent launch): the step kernels wait for it on the device
 // (grid_dependency_wait) before they touch memory it writes, so only the
 // launch and the shared-memory set-up overlap.  Measured on 400 x 1200 with
 // one shot, the forward runs 6 % faster; with 32 shots nothing changes.
-cudaError_t launch_pdl(const void *fn, dim3 grid, size_t smem, void **args, cudaStream_t st)
+cudaError_t launch_kernel(gb_plan *P, const void *fn, dim3 grid, dim3 block, size_t smem, void **args, cudaStream_t st,
+                          bool pdl)
 {
+    if (P->updating) {
+        if (P->next_node >= P->updating->nodes.size()) return cudaErrorInvalidValue;
+        cudaKernelNodeParams np = {};
+        np.func = const_cast<void *>(fn);
+        np.gridDim = grid;
+        np.blockDim = block;
+        np.sharedMemBytes = (unsigned)smem;
+        np.kernelParams = args;
+        return cudaGraphExecKernelNodeSetParams(P->updating->exec, P->updating->nodes[P->next_node++], &np);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(NTHR);
+    cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelExC(&cfg, fn, args);
+    if (pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+    if (e != cudaSuccess || !P->recording) return e;
+    // the node just captured is the stream's one dependency
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t n = 0;
+    const cudaError_t q = cudaStreamGetCaptureInfo_v3(st, &status, nullptr, nullptr, &deps, &edges, &n);
+    if (q != cudaSuccess) return q;
+    if (n != 1) return cudaErrorStreamCaptureUnmatched;
+    P->recording->nodes.push_back(deps[0]);
+    return cudaSuccess;
+}
+
+cudaError_t launch_pdl(gb_plan *P, const void *fn, dim3 grid, size_t smem, void **args, cudaStream_t st)
+{
+    return launch_kernel(P, fn, grid, dim3(NTHR), smem, args, st, true);
 }
 
 // The CTA schedule of a launch of groups [grp0, grp0 + grp_count): the
@@ -609,7 +650,7 @@ int launch_step(gb_plan *P, const StepKernel &K, const Maps &maps, Args A, int g
     apply_schedule(P, A, grp0, grp_count, &grid);
     void *args[] = {(void *)&maps.p, (void *)&maps.vx, (void *)&maps.vz, (void *)&maps.a1, (void *)&maps.a2,
                     (void *)&A};
-    GB_CUDA(launch_pdl(K.fn, dim3(grid), K.smem, args, st));
+    GB_CUDA(launch_pdl(P, K.fn, dim3(grid), K.smem, args, st));
     ++P->launches;
     ++P->api_launches;
     return GB_OK;
@@ -628,14 +669,14 @@ int launch_step(gb_plan *P, const StepKernel &K, const Maps &maps, FwdArgs A, in
     SA.n_seg = (P->tiles_z + SA.seg_chunks - 1) / SA.seg_chunks;
     void *args[] = {(void *)&maps.sp,  (void *)&maps.svx, (void *)&maps.svz, (void *)&maps.sa1,
                     (void *)&maps.sa2, (void *)&A,         (void *)&SA};
-    GB_CUDA(launch_pdl(K.fn, dim3((unsigned)P->tiles_x * SA.n_seg * SA.n_shots), K.smem, args, st));
+    GB_CUDA(launch_pdl(P, K.fn, dim3((unsigned)P->tiles_x * SA.n_seg * SA.n_shots), K.smem, args, st));
     ++P->launches;
     ++P->api_launches;
     return GB_OK;
 }
 
-// Streams the shot groups run on: the caller's stream when there is one
-// group (or grouping is off), else one stream per group forked from it.
+// Streams the shot groups run on: the caller's stream when there is one lane
+// (or group streams are off), else one stream per lane forked from it.
 struct GroupStreams {
     gb_plan *P;
     cudaStream_t main;
@@ -644,13 +685,20 @@ struct GroupStreams {
     cudaStream_t at(int grp) const { return n == 1 ? main : P->gstream[grp]; }
 };
 
-// want < 0: one stream per shot group when group streams are on; else
-// `want` streams (the lanes of a batch)
+// Lanes the shot groups of a plan run in: neighbouring groups share one, a
+// launch a step each.
+constexpr int kGroupLanes = 4;
+int group_lanes(const gb_plan *P)
+{
+    return P->group_streams ? std::max(1, std::min(P->n_groups, kGroupLanes)) : 1;
+}
+
+// want < 0: the lanes of the plan's groups; else `want` streams (the lanes of a batch)
 int group_streams(gb_plan *P, cudaStream_t main, GroupStreams *gs, int want = -1)
 {
     gs->P = P;
     gs->main = main;
-    gs->n = want >= 0 ? std::max(1, want) : (P->group_streams && P->n_groups > 1) ? P->n_groups : 1;
+    gs->n = want >= 0 ? std::max(1, want) : group_lanes(P);
     if (gs->n == 1) return GB_OK;
     int dev = -1;
     GB_CUDA(cudaGetDevice(&dev));
@@ -688,116 +736,103 @@ int join(const GroupStreams &gs)
     return GB_OK;
 }
 
-// groups handled by one launch on stream i: all of them on a single stream
+// groups handled by one launch on stream i: an even share of them
 inline void launch_groups(const GroupStreams &gs, int i, int n_groups, int *g0, int *gc)
 {
-    if (gs.n == 1) {
-        *g0 = 0;
-        *gc = n_groups;
-    } else {
-        *g0 = i;
-        *gc = 1;
-    }
+    *g0 = (int)((long long)n_groups * i / gs.n);
+    *gc = (int)((long long)n_groups * (i + 1) / gs.n) - *g0;
+}
+
+// the shots of groups [g0, g0 + gc)
+inline void lane_shots(const gb_plan *P, int g0, int gc, int *s0, int *ns)
+{
+    *s0 = P->group_first(g0);
+    *ns = std::min(P->d.n_shots, P->group_first(g0 + gc)) - *s0;
 }
 
 // ---------------------------------------------------------------------------
-// CUDA graph of a chunk of plain forward steps.  The graph holds C steps of
-// every shot group (C even, so step j of the chunk reads state level j & 1)
-// with the group fork / join, then advances a device step counter by C; the
-// step kernels take their step index from that counter.  It is captured once
-// for a given set of buffers and replayed nt / C times.
+// CUDA graphs of chunks of steps.  A graph holds C steps of every lane (C
+// even, so step j of the chunk reads state level j & 1) with the lanes' fork
+// and join, then advances a device step counter; the step kernels take their
+// step index from that counter, so one graph serves every chunk of a loop.
 // ---------------------------------------------------------------------------
 constexpr int kMaxGraphSteps = 64;
 
-int capture_forward_chunk(gb_plan *P, const StepKernel &K, const Maps (&maps)[2], float *const (&buf)[2],
-                          float *const (&psi)[2], FwdArgs A, int C, int *step_ctr, cudaGraphExec_t *out)
-{
-    GroupStreams gs;
-    if (int rc = group_streams(P, nullptr, &gs)) return rc;      // (re)creating the group streams drops cap_stream
-    if (!P->cap_stream) GB_CUDA(cudaStreamCreateWithFlags(&P->cap_stream, cudaStreamNonBlocking));
-    gs.main = P->cap_stream;
-    const long long launches = P->launches;
-    GB_CUDA(cudaStreamBeginCapture(P->cap_stream, cudaStreamCaptureModeThreadLocal));
-    int rc = fork(gs);
-    A.step_base = step_ctr;
-    for (int j = 0; j < C && rc == GB_OK; ++j) {
-        A.it = j;
-        A.out = buf[(j & 1) ^ 1];
-        if (A.cpml) {
-            A.psi_in = psi[j & 1];
-            A.psi_out = psi[(j & 1) ^ 1];
-        }
-        for (int i = 0; i < gs.n && rc == GB_OK; ++i) {
-            int g0, gc;
-            launch_groups(gs, i, P->n_groups, &g0, &gc);
-            rc = launch_step(P, K, maps[j & 1], A, g0, gc, gs.at(i));
-        }
-    }
-    if (rc == GB_OK) rc = join(gs);
-    if (rc == GB_OK) {
-        step_advance_kernel<<<1, 1, 0, P->cap_stream>>>(step_ctr, C);
-        if (cudaGetLastError() != cudaSuccess) rc = fail(GB_E_CUDA, "graph capture: launch failed");
-    }
-    cudaGraph_t graph = nullptr;
-    const cudaError_t ec = cudaStreamEndCapture(P->cap_stream, &graph);   // always end the capture
-    P->launches = launches;
-    if (rc != GB_OK) {
-        if (graph) cudaGraphDestroy(graph);
-        return rc;
-    }
-    if (ec != cudaSuccess) return fail(GB_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(ec));
-    const cudaError_t ei = cudaGraphInstantiate(out, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ei != cudaSuccess) return fail(GB_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ei));
-    return GB_OK;
-}
-
-// Capture `C` steps of a step loop into `slot` (unless it already holds a
-// graph for `key`): launch(j, gs) launches step j of the chunk on the group
-// streams gs, and after the steps the device counter ctr moves by `advance`;
-// the step kernels read their step index from that counter.
+// Make `slot` hold `C` steps of a step loop: launch(j, gs) launches step j of
+// the chunk on the streams gs, and after the steps the device counter ctr
+// moves by `advance`.  Captured once per `key`; with other `args` the nodes of
+// the graph that is there get their parameters from the same launches.
 template <class Launch>
-int capture_chunk(gb_plan *P, gb_plan::GraphSlot &slot, const std::vector<uintptr_t> &key, int C, int *ctr,
-                  int advance, bool group_streams_on, Launch launch, int n_streams = -1)
+int capture_chunk(gb_plan *P, gb_plan::GraphSlot &slot, const std::vector<uintptr_t> &key,
+                  const std::vector<uintptr_t> &args, int C, int *ctr, int advance, bool group_streams_on,
+                  Launch launch, int n_streams = -1)
 {
-    if (slot.exec && slot.key == key) return GB_OK;
-    slot.release();
+    const bool reuse = slot.exec && slot.key == key;
+    if (reuse && slot.args == args) return GB_OK;
+    if (!reuse) slot.release();
     GroupStreams gs;
     if (group_streams_on) {
-        // (re)creating the group streams drops cap_stream
+        // (re)creating the streams drops cap_stream and every graph
         if (int rc = group_streams(P, nullptr, &gs, n_streams)) return rc;
     } else {
         gs.P = P;
         gs.n = 1;
     }
+    if (reuse && !slot.exec) return capture_chunk(P, slot, key, args, C, ctr, advance, group_streams_on, launch, n_streams);
     if (!P->cap_stream) GB_CUDA(cudaStreamCreateWithFlags(&P->cap_stream, cudaStreamNonBlocking));
     gs.main = P->cap_stream;
     const long long launches = P->launches, api = P->api_launches;
-    GB_CUDA(cudaStreamBeginCapture(P->cap_stream, cudaStreamCaptureModeThreadLocal));
-    int rc = group_streams_on ? fork(gs) : GB_OK;
-    for (int j = 0; j < C && rc == GB_OK; ++j) rc = launch(j, gs);
-    if (rc == GB_OK && group_streams_on) rc = join(gs);
-    if (rc == GB_OK) {
-        step_advance_kernel<<<1, 1, 0, P->cap_stream>>>(ctr, advance);
-        if (cudaGetLastError() != cudaSuccess) rc = fail(GB_E_CUDA, "graph capture: launch failed");
+    auto steps = [&]() -> int {
+        int rc = GB_OK;
+        for (int j = 0; j < C && rc == GB_OK; ++j) rc = launch(j, gs);
+        return rc;
+    };
+    auto advance_step = [&]() -> int {
+        int *c = ctr, by = advance;
+        void *a[] = {(void *)&c, (void *)&by};
+        GB_CUDA(launch_kernel(P, (const void *)&step_advance_kernel, dim3(1), dim3(1), 0, a, P->cap_stream, false));
+        return GB_OK;
+    };
+    if (reuse) {
+        P->updating = &slot;
+        P->next_node = 0;
+        int rc = steps();
+        if (rc == GB_OK) rc = advance_step();
+        const bool all = P->next_node == slot.nodes.size();
+        P->updating = nullptr;
+        P->launches = launches;
+        P->api_launches = api;
+        if (rc == GB_OK && all) {
+            slot.args = args;
+            return GB_OK;
+        }
+        cudaGetLastError();
+        slot.release();                      // captured afresh below
     }
+    GB_CUDA(cudaStreamBeginCapture(P->cap_stream, cudaStreamCaptureModeThreadLocal));
+    P->recording = &slot;
+    int rc = group_streams_on ? fork(gs) : GB_OK;
+    if (rc == GB_OK) rc = steps();
+    if (rc == GB_OK && group_streams_on) rc = join(gs);
+    if (rc == GB_OK) rc = advance_step();
+    P->recording = nullptr;
     cudaGraph_t graph = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(P->cap_stream, &graph);   // always end the capture
     P->launches = launches;
     P->api_launches = api;
-    if (rc != GB_OK) {
-        if (graph) cudaGraphDestroy(graph);
-        return rc;
+    slot.graph = graph;
+    cudaError_t ei = cudaSuccess;
+    if (rc == GB_OK && ec == cudaSuccess) ei = cudaGraphInstantiate(&slot.exec, graph, 0);
+    if (rc == GB_OK && ec == cudaSuccess && ei == cudaSuccess) {
+        slot.key = key;
+        slot.args = args;
+        return GB_OK;
     }
+    if (ei != cudaSuccess) slot.exec = nullptr;
+    slot.release();
+    if (rc != GB_OK) return rc;
     if (ec != cudaSuccess) return fail(GB_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(ec));
-    const cudaError_t ei = cudaGraphInstantiate(&slot.exec, graph, 0);
-    cudaGraphDestroy(graph);
-    if (ei != cudaSuccess) {
-        slot.exec = nullptr;
-        return fail(GB_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ei));
-    }
-    slot.key = key;
-    return GB_OK;
+    return fail(GB_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ei));
 }
 
 // Per-checkpoint sizes of the 16-bit formats.
@@ -1538,21 +1573,35 @@ int gb_forward(gb_plan *P, const float *vp, const float *rho, const float *damp,
         int *step_ctr = reinterpret_cast<int *>(ws + L.err + 128);
         int dev = -1;
         GB_CUDA(cudaGetDevice(&dev));
-        const std::vector<uintptr_t> key = {
-            (uintptr_t)dev, (uintptr_t)ws, (uintptr_t)wavelet, (uintptr_t)trace_p, (uintptr_t)trace_vx,
-            (uintptr_t)trace_vz, (uintptr_t)want_energy, (uintptr_t)C, (uintptr_t)P->tz, (uintptr_t)P->spc_eff,
-            (uintptr_t)P->n_groups, (uintptr_t)gs.n, (uintptr_t)K0.fn, (uintptr_t)P->sched};
-        if (!P->gexec || P->gkey != key) {
-            P->release_graph();
-            if (int rc = capture_forward_chunk(P, K0, maps, buf, Su.psi, A, C, step_ctr, &P->gexec)) return rc;
-            P->gkey = key;
-        }
+        const std::vector<uintptr_t> key = {(uintptr_t)dev, (uintptr_t)K0.fn, (uintptr_t)C, (uintptr_t)gs.n};
+        const std::vector<uintptr_t> args = {
+            (uintptr_t)ws, (uintptr_t)wavelet, (uintptr_t)trace_p, (uintptr_t)trace_vx, (uintptr_t)trace_vz,
+            (uintptr_t)want_energy, (uintptr_t)P->tz, (uintptr_t)P->spc_eff, (uintptr_t)P->n_groups,
+            (uintptr_t)P->sched, (uintptr_t)d.nt};
+        FwdArgs B = A;
+        B.step_base = step_ctr;
+        if (int rc = capture_chunk(P, P->g_fwd, key, args, C, step_ctr, C, true, [&](int j, const GroupStreams &g) {
+                FwdArgs Bj = B;
+                Bj.it = j;
+                Bj.out = buf[(j & 1) ^ 1];
+                if (Su.cpml) {
+                    Bj.psi_in = Su.psi[j & 1];
+                    Bj.psi_out = Su.psi[(j & 1) ^ 1];
+                }
+                for (int i = 0; i < g.n; ++i) {
+                    int g0, gc;
+                    launch_groups(g, i, P->n_groups, &g0, &gc);
+                    if (int rc = launch_step(P, K0, maps[j & 1], Bj, g0, gc, g.at(i))) return rc;
+                }
+                return (int)GB_OK;
+            }))
+            return rc;
         step_set_kernel<<<1, 1, 0, st>>>(step_ctr, 0);
         GB_CUDA(cudaGetLastError());
         ++P->launches;
         const int n_chunks = d.nt / C;
         for (int k = 0; k < n_chunks; ++k) {
-            GB_CUDA(cudaGraphLaunch(P->gexec, st));
+            GB_CUDA(cudaGraphLaunch(P->g_fwd.exec, st));
             P->launches += (long long)C * gs.n + 1;
             ++P->api_launches;
             const int last = (k + 1) * C - 1;
@@ -1581,8 +1630,8 @@ int gb_forward(gb_plan *P, const float *vp, const float *rho, const float *damp,
             launch_groups(gs, i, P->n_groups, &g0, &gc);
             const cudaStream_t si = gs.at(i);
             if (store && it < t_cache && it % K == 0) {
-                const int s0 = P->group_first(g0);
-                const int ns = gs.n == 1 ? S : P->group_shots(g0);
+                int s0, ns;
+                lane_shots(P, g0, gc, &s0, &ns);
                 if (int rc = save_checkpoint(P, buf[b], store->checkpoints, it / K, store->format, Su.amax, s0, ns, si))
                     return rc;
             }
@@ -1609,18 +1658,19 @@ int gb_forward(gb_plan *P, const float *vp, const float *rho, const float *damp,
             int *step_ctr = reinterpret_cast<int *>(ws + L.err + 128);
             int dev = -1;
             GB_CUDA(cudaGetDevice(&dev));
-            const std::vector<uintptr_t> key = {
-                (uintptr_t)dev, (uintptr_t)ws, (uintptr_t)wavelet, (uintptr_t)trace_p, (uintptr_t)trace_vx,
-                (uintptr_t)trace_vz, (uintptr_t)want_energy, (uintptr_t)C, (uintptr_t)P->tz, (uintptr_t)P->spc_eff,
-                (uintptr_t)P->n_groups, (uintptr_t)gs.n, (uintptr_t)KI.fn, (uintptr_t)store->imaging,
-                (uintptr_t)t_cache, (uintptr_t)store->imaging_format, (uintptr_t)store->with_rho, (uintptr_t)P->sched};
+            const std::vector<uintptr_t> key = {(uintptr_t)dev, (uintptr_t)KI.fn, (uintptr_t)C, (uintptr_t)gs.n};
+            const std::vector<uintptr_t> args = {
+                (uintptr_t)ws, (uintptr_t)wavelet, (uintptr_t)trace_p, (uintptr_t)trace_vx, (uintptr_t)trace_vz,
+                (uintptr_t)want_energy, (uintptr_t)P->tz, (uintptr_t)P->spc_eff, (uintptr_t)P->n_groups,
+                (uintptr_t)store->imaging, (uintptr_t)t_cache, (uintptr_t)store->imaging_format,
+                (uintptr_t)store->with_rho, (uintptr_t)P->sched, (uintptr_t)d.nt};
             FwdArgs B = A;
             B.step_base = step_ctr;
             B.img_base = reinterpret_cast<float *>(store->imaging);
             B.img_step = (long long)step_img;
             B.img_t0 = t_cache;
             B.imaging = reinterpret_cast<float *>(store->imaging);
-            if (int rc = capture_chunk(P, P->g_fwd_img, key, C, step_ctr, C, true, [&](int j, const GroupStreams &g) {
+            if (int rc = capture_chunk(P, P->g_fwd_img, key, args, C, step_ctr, C, true, [&](int j, const GroupStreams &g) {
                     FwdArgs Bj = B;
                     Bj.it = j;
                     Bj.out = buf[(j & 1) ^ 1];
@@ -1947,18 +1997,19 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
                 if (int rc = join(gs)) return rc;
                 int dev = -1;
                 GB_CUDA(cudaGetDevice(&dev));
-                const std::vector<uintptr_t> key = {
-                    (uintptr_t)dev, (uintptr_t)ws, (uintptr_t)res_p, (uintptr_t)res_vx, (uintptr_t)res_vz,
-                    (uintptr_t)img_base, (uintptr_t)img_fmt, (uintptr_t)t0, (uintptr_t)grad_wavelet, (uintptr_t)C,
-                    (uintptr_t)P->tz, (uintptr_t)P->spc_eff, (uintptr_t)P->n_groups, (uintptr_t)gs.n,
-                    (uintptr_t)KA.fn, (uintptr_t)rho_fields, (uintptr_t)P->sched};
+                const std::vector<uintptr_t> key = {(uintptr_t)dev, (uintptr_t)KA.fn, (uintptr_t)C, (uintptr_t)gs.n};
+                const std::vector<uintptr_t> args = {
+                    (uintptr_t)ws, (uintptr_t)res_p, (uintptr_t)res_vx, (uintptr_t)res_vz, (uintptr_t)img_base,
+                    (uintptr_t)img_fmt, (uintptr_t)t0, (uintptr_t)grad_wavelet, (uintptr_t)P->tz,
+                    (uintptr_t)P->spc_eff, (uintptr_t)P->n_groups, (uintptr_t)rho_fields, (uintptr_t)P->sched,
+                    (uintptr_t)d.nt};
                 AdjArgs B = A;
                 B.step_base = step_ctr;
                 B.img_base = reinterpret_cast<float *>(img_base);
                 B.img_step = (long long)step_img;
                 B.img_t0 = t0;
                 B.img_fmt = img_fmt;
-                if (int rc = capture_chunk(P, P->g_adj, key, C, step_ctr, -C, true, [&](int j, const GroupStreams &g) {
+                if (int rc = capture_chunk(P, P->g_adj, key, args, C, step_ctr, -C, true, [&](int j, const GroupStreams &g) {
                         AdjArgs Bj = B;
                         Bj.it = j;
                         Bj.out = mu[(j & 1) ^ 1];
@@ -2003,7 +2054,8 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
         for (int i = 0; i < gs.n; ++i) {
             int g0, gc;
             launch_groups(gs, i, P->n_groups, &g0, &gc);
-            const int s0 = P->group_first(g0), ns = gs.n == 1 ? S : P->group_shots(g0);
+            int s0, ns;
+            lane_shots(P, g0, gc, &s0, &ns);
             if (int rc = restore_checkpoint(P, fb[0], store->checkpoints, seg, store->format, s0, ns, gs.at(i)))
                 return rc;
         }
@@ -2180,7 +2232,7 @@ int make_state_maps(const gb_plan *P, const float *buf, CUtensorMap (&m)[3])
 
 int launch_batch(gb_plan *P0, const StepKernel &K, long long n_items, void **args, cudaStream_t st)
 {
-    GB_CUDA(cudaLaunchKernel(K.fn, dim3((unsigned)n_items), dim3(NTHR), args, K.smem, st));
+    GB_CUDA(launch_kernel(P0, K.fn, dim3((unsigned)n_items), dim3(NTHR), K.smem, args, st, false));
     ++P0->launches;
     ++P0->api_launches;
     return GB_OK;
@@ -2220,16 +2272,28 @@ BatchLanes batch_lanes(gb_plan *const *plans, int n_models, long long n_items)
     return L;
 }
 
+// What the arguments of a batch's launches are made of: its workspace (with
+// n models' tables laid out in it) and the lanes' runs of items.
+std::vector<uintptr_t> lane_args(const char *bws, int n, const BatchLanes &lanes)
+{
+    std::vector<uintptr_t> a = {(uintptr_t)bws, (uintptr_t)n};
+    for (int i = 0; i < lanes.n; ++i) {
+        a.push_back((uintptr_t)lanes.off[i]);
+        a.push_back((uintptr_t)lanes.cnt[i]);
+    }
+    return a;
+}
+
 // A batched step loop in chunks of C steps replayed from the CUDA graph in
 // `slot` (captured once per key): launch(j, lane, stream) launches step j of
 // a chunk for one lane, the kernels reading the batch clock at `clock`,
 // which starts at `first` and moves by `dir` * C after each chunk.
 template <class Launch>
-int batch_graph_chunks(gb_plan *P0, gb_plan::GraphSlot &slot, const std::vector<uintptr_t> &key, int C, int *clock,
-                       int first, int dir, int n_chunks, const BatchLanes &lanes, cudaStream_t st, Launch launch)
+int batch_graph_chunks(gb_plan *P0, gb_plan::GraphSlot &slot, const std::vector<uintptr_t> &key,
+                       const std::vector<uintptr_t> &args, int C, int *clock, int first, int dir, int n_chunks, const BatchLanes &lanes, cudaStream_t st, Launch launch)
 {
     if (int rc = capture_chunk(
-            P0, slot, key, C, clock, dir * C, lanes.n > 1,
+            P0, slot, key, args, C, clock, dir * C, lanes.n > 1,
             [&](int j, const GroupStreams &g) {
                 for (int i = 0; i < lanes.n; ++i)
                     if (int rc = launch(j, i, lanes.n > 1 ? g.at(i) : g.main)) return rc;
@@ -2344,8 +2408,8 @@ int gb_batch_forward(gb_plan *const *plans, int n, const gb_model_io *io, void *
     int dev = -1;
     GB_CUDA(cudaGetDevice(&dev));
     const BatchLanes lanes = batch_lanes(plans, n, B.n_items);
-    const std::vector<uintptr_t> key = {(uintptr_t)dev, (uintptr_t)bws, (uintptr_t)B.n_items, (uintptr_t)K0.fn,
-                                        (uintptr_t)C, (uintptr_t)kBatchForward, (uintptr_t)lanes.n};
+    const std::vector<uintptr_t> key = {(uintptr_t)dev, (uintptr_t)K0.fn, (uintptr_t)C, (uintptr_t)lanes.n};
+    const std::vector<uintptr_t> gargs = lane_args(bws, n, lanes);
     for (int tau = 0; tau < maxnt;) {
         for (int m = 0; m < n; ++m) {
             const gb_grad_store *sto = io[m].store;
@@ -2369,7 +2433,7 @@ int gb_batch_forward(gb_plan *const *plans, int n, const gb_model_io *io, void *
                 ++n_chunks;
             }
         if (n_chunks > 0) {
-            if (int rc = batch_graph_chunks(P0, P0->g_batch_fwd, key, C, clock, tau, 1, n_chunks, lanes, st,
+            if (int rc = batch_graph_chunks(P0, P0->g_batch_fwd, key, gargs, C, clock, tau, 1, n_chunks, lanes, st,
                                             [&](int j, int lane, cudaStream_t s2) {
                                                 int tau_v = j;
                                                 const int4 *it_l = items + lanes.off[lane];
@@ -2511,8 +2575,8 @@ int gb_batch_backward(gb_plan *const *plans, int n, const gb_model_io *io, void 
     int dev = -1;
     GB_CUDA(cudaGetDevice(&dev));
     const BatchLanes lanes = batch_lanes(plans, n, B.n_items);
-    const std::vector<uintptr_t> akey = {(uintptr_t)dev, (uintptr_t)bws, (uintptr_t)B.n_items, (uintptr_t)KA.fn,
-                                         (uintptr_t)C, (uintptr_t)lanes.n};
+    const std::vector<uintptr_t> akey = {(uintptr_t)dev, (uintptr_t)KA.fn, (uintptr_t)C, (uintptr_t)lanes.n};
+    const std::vector<uintptr_t> gargs = lane_args(bws, n, lanes);
     // batch-wide segments of K steps; a model recomputes a segment only for
     // its steps below min(nt, t_cache)
     const int Kb = std::min(K, maxnt);
@@ -2548,7 +2612,7 @@ int gb_batch_backward(gb_plan *const *plans, int n, const gb_model_io *io, void 
         // chunks of C steps replayed from one graph (the clock counts down)
         const int n_chunks = C > 0 ? (t1 - t0) / C : 0;
         if (n_chunks > 0) {
-            if (int rc = batch_graph_chunks(P0, P0->g_batch_adj, akey, C, clock, tau, -1, n_chunks, lanes, st,
+            if (int rc = batch_graph_chunks(P0, P0->g_batch_adj, akey, gargs, C, clock, tau, -1, n_chunks, lanes, st,
                                             [&](int j, int lane, cudaStream_t s2) {
                                                 int tau_v = j;
                                                 const int4 *it_l = items + lanes.off[lane];
