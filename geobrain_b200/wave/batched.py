@@ -282,6 +282,17 @@ def full_cache_bytes(plan, with_rho: bool, imaging_dtype: str) -> int:
             plan.gradient_workspace_bytes(with_rho, 1, imaging_dtype) + 4 * S * nt * NR * 4)
 
 
+def batch_hold_bytes(plans, with_rho: bool, imaging_dtype: str) -> int:
+    """Device bytes a fused batched gradient of these models holds at once, at
+    its fullest: the imaging fields, the larger of the forward's and the
+    adjoint's workspaces (one is given back before the other is taken) and
+    two trace fields."""
+    img = sum(_align256(p.imaging_bytes(p.geo.nt, with_rho, imaging_dtype)) for p in plans)
+    fwd = sum(p.workspace_bytes(False, 0) for p in plans)
+    adj = sum(p.gradient_workspace_bytes(with_rho, 1, imaging_dtype) for p in plans)
+    return img + max(fwd, adj) + sum(2 * p.n_shots * p.geo.nt * p.n_rcv * 4 for p in plans)
+
+
 def plan_sub_batches(sizes: Sequence[int], avail: int) -> List[List[int]]:
     """Split models (in order) into consecutive sub-batches whose summed
     sizes fit in `avail` bytes, as few as fit and as even as they can be: a
@@ -353,13 +364,16 @@ def acoustic_gradient_batched(models: Sequence[dict], residual, *, fd_order: int
     n = len(prep.plans)
     vps = [_as_f32(m["vp"].detach() if torch.is_tensor(m["vp"]) else m["vp"], device, "vp") for m in models]
     rhos = [_as_f32(m["rho"].detach() if torch.is_tensor(m["rho"]) else m["rho"], device, "rho") for m in models]
+    sizes = [full_cache_bytes(p, with_rho, imaging_dtype) for p in prep.plans]
+    pool = engine.unused_pool(device)
     if memory_budget is not None:
         avail = int(memory_budget)
+    elif batch_hold_bytes(prep.plans, with_rho, imaging_dtype) <= pool:
+        avail = sum(sizes)               # one sub-batch, out of what the allocator holds unused
     else:
         free, _ = torch.cuda.mem_get_info(device)
-        avail = free + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+        avail = free + pool
         avail -= (2 << 30) + avail // 20
-    sizes = [full_cache_bytes(p, with_rho, imaging_dtype) for p in prep.plans]
     losses = torch.zeros(n, dtype=torch.float32, device=device)
     grads_vp, grads_rho = [None] * n, [None] * n
     L = _bind()

@@ -302,6 +302,14 @@ def choose_checkpoint_every(plan: Plan, checkpoint_segments: int = 1, checkpoint
     return max(1, min(k, nt))
 
 
+def unused_pool(device) -> int:
+    """Bytes torch's caching allocator holds on the device and does not use:
+    memory that is there for certain, known without asking the driver
+    (cudaMemGetInfo took between 0.1 and 70 ms a call on a shared host,
+    against 2 ms for the rest of a gradient's host work)."""
+    return torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+
+
 def choose_cached_steps(plan: Plan, imaging_cache, with_rho: bool, device, imaging_fmt: str = "fp32",
                         checkpoint_every: int = 1, ckpt_fmt: str = "fp32", memory_budget: Optional[int] = None) -> int:
     """How many of the last time steps keep their imaging fields from the
@@ -323,20 +331,32 @@ def choose_cached_steps(plan: Plan, imaging_cache, with_rho: bool, device, imagi
     env = os.environ.get("GEOBRAIN_B200_IMAGING_CACHE_BYTES")
     if env is not None:
         return int(max(0, min(nt, int(env) // per)))
-    free, _ = torch.cuda.mem_get_info(device)
-    # blocks torch's allocator holds but does not use are free for this too
-    avail = free + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
-    if memory_budget is not None:
-        avail = min(avail, int(memory_budget))
     K = max(1, min(int(checkpoint_every), nt))
     one_ck = plan.checkpoint_bytes(nt, ckpt_fmt)                      # one stored state
-    fixed = 3 * plan.n_shots * nt * plan.n_rcv * 4 + (2 << 30) + avail // 20
+    traces = 3 * plan.n_shots * nt * plan.n_rcv * 4
 
-    def need(c: int) -> int:
+    def hold(c: int) -> int:
         rest = nt - c
         seg = max(1, min(K, rest))
         return (c * per + -(-rest // K) * one_ck + plan.gradient_workspace_bytes(with_rho, seg, imaging_fmt) +
-                plan.workspace_bytes(0, 0) + fixed)
+                plan.workspace_bytes(0, 0) + traces)
+
+    # every step's fields, the larger of the two workspaces (the forward's is
+    # given back before the adjoint's is taken) and a trace field fit in what
+    # the allocator holds unused, as after an earlier call: no need to ask
+    pool = unused_pool(device)
+    if memory_budget is None and nt * per + max(plan.workspace_bytes(0, 0),
+                                                plan.gradient_workspace_bytes(with_rho, 1, imaging_fmt)) + traces // 3 <= pool:
+        return nt
+    free, _ = torch.cuda.mem_get_info(device)
+    # blocks torch's allocator holds but does not use are free for this too
+    avail = free + pool
+    if memory_budget is not None:
+        avail = min(avail, int(memory_budget))
+    margin = (2 << 30) + avail // 20
+
+    def need(c: int) -> int:
+        return hold(c) + margin
 
     if need(nt) <= avail:                # no recompute at all (no segment buffer either)
         return nt

@@ -83,10 +83,14 @@ class _Run3:
 def _imaging_fits(run, nbytes: int) -> bool:
     """Whether nbytes of imaging fields, the adjoint's workspace and a margin
     (2 GiB + 5 %) fit in the device memory available now (counting blocks the
-    caching allocator holds unused)."""
-    free, _ = torch.cuda.mem_get_info(run.device)
-    avail = free + torch.cuda.memory_reserved(run.device) - torch.cuda.memory_allocated(run.device)
+    caching allocator holds unused, which alone are enough after an earlier
+    call: the driver is asked only when they are not)."""
     ws = int(run.L.gb3_backward_workspace_bytes(ctypes.byref(run.desc), 0, 1))
+    pool = engine.unused_pool(run.device)
+    if nbytes + ws + 4 * run.desc.n_shots * run.desc.nt * run.desc.n_rcv <= pool:
+        return True
+    free, _ = torch.cuda.mem_get_info(run.device)
+    avail = free + pool
     return nbytes + ws + (2 << 30) + avail // 20 <= avail
 
 
