@@ -322,22 +322,31 @@ __global__ void rec3_kernel(const Geo3 g, const float *state, const int *rcv, fl
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint (reverse time) of one step, in gather form.  lam = adjoint of the
-// state after the step; the two kernels below undo the velocity updates and
-// then the pressure update:
-//   adj_v3: lp' = lp + sum_c -G_c^T (a2 lam_c on M_c),  lam_c' = (1 - k_c) lam_c on M_c
-//   adj_p3: lp  = (1 - k1) lp' on M_p,  lam_c = lam_c' - D_c^T (a1 lp' on M_p)
-// with (G^T w)[q] = c1 (w[q-1] - w[q]) + c2 (w[q-2] - w[q+1]) and
-// (D^T u)[q] = c1 (u[q] - u[q+1]) + c2 (u[q-1] - u[q+2]) along each
-// component's axis, and the gradient sums dL/da1 += lp' I, dL/da2 +=
-// -lam_c J_c (Neumaier-compensated, one owner per cell, no atomics).
+// Adjoint (reverse time) of one step, in the scaled variables mu_p = a1 lam_p
+// and mu_c = a2 lam_c (lam: the adjoint of the state).  In those the adjoint
+// has the forward's shape, and each kernel reads only its own cell's
+// coefficients and updates in place, as the forward's do:
+//   inject   mu_c[receiver] += a2 dL/dtrace_c
+//   adj_p3   mu_p  <- (1 - k1) mu_p + a1 (div mu_v)                (p mask)
+//   inject   mu_p[receiver] += a1 dL/dtrace_p
+//   adj_v3   G1 += mu_p I,  G2 += sum_c mu_c J_c,
+//            mu_c  <- (1 - k_c) mu_c + a2 d_c(mu_p)               (mask of c)
+// The damping of mu_p belongs to the end of the step: it is applied when the
+// next step reads the value, so that adj_v3's neighbours see it undamped.
+// Cells off the masks never depend on the model; their adjoint is dropped
+// (held at zero), which keeps every stencil read mask-free.  Free surface: the
+// mirror planes p[fs-1] = -p[fs+1] and vz[fs-1] = vz[fs] hand their share to
+// planes fs + 1 and fs; with all off-mask cells at zero each share is one term.
+// Unscaled, in gather form with two state buffers, the two kernels held 28
+// neighbour coefficients a thread and moved 68 bytes per cell and shot: 449 us
+// a step at 166 x 185 x 207 with 4 shots.
 // ---------------------------------------------------------------------------
 struct AdjArgs3 {
     Geo3 g;
-    const float *lam_in;          // [S][4][vol] adjoint state
-    float *lam_out;
+    int free_surface;
+    float *mu;                    // [S][4][vol] adjoint state, updated in place
     const float *a1, *k1, *a2, *k2, *k3, *k4;
-    const float *img_i, *img_j;   // this step's recomputed imaging fields
+    const float *img_i, *img_j;   // this step's imaging fields
     float *G1, *C1, *G2, *C2;     // [vol] gradient sums and compensations (G2 / C2 null without density)
 };
 
@@ -351,10 +360,9 @@ __device__ __forceinline__ void neumaier3(float &s, float &c, float x)
     s = t;
 }
 
-__device__ __forceinline__ bool in_px(const Geo3 &g, int x) { return x >= 2 && x < g.Nx - 2; }
 __device__ __forceinline__ bool in_p(const Geo3 &g, int z, int y, int x)
 {
-    return z >= g.fs + 1 && z < g.Nz - 2 && y >= 2 && y < g.Ny - 2 && in_px(g, x);
+    return z >= g.fs + 1 && z < g.Nz - 2 && y >= 2 && y < g.Ny - 2 && x >= 2 && x < g.Nx - 2;
 }
 __device__ __forceinline__ bool in_vx(const Geo3 &g, int z, int y, int x)
 {
@@ -368,238 +376,210 @@ __device__ __forceinline__ bool in_vz(const Geo3 &g, int z, int y, int x)
 {
     return z >= g.fs && z < g.Nz - 2 && y >= 1 && y < g.Ny - 1 && x >= 1 && x < g.Nx - 1;
 }
-// value at (z, y, x) of field f, 0 outside the grid
-__device__ __forceinline__ float at3(const Geo3 &g, const float *F, int z, int y, int x)
-{
-    if (z < 0 || z >= g.Nz || y < 0 || y >= g.Ny || x < 0 || x >= g.Nx) return 0.f;
-    return F[(long long)z * g.plane + (long long)y * g.pitch + x];
-}
 
-// float4 of field F at (z, y, x4), 0 outside the grid rows / planes; x4 is a
-// multiple of 4 and x4 - 4 >= 0 is checked by the caller's guard
-__device__ __forceinline__ float4 row4(const Geo3 &g, const float *F, int z, int y, int x4)
-{
-    if (z < 0 || z >= g.Nz || y < 0 || y >= g.Ny || x4 < 0 || x4 >= g.pitch) return make_float4(0.f, 0.f, 0.f, 0.f);
-    return *reinterpret_cast<const float4 *>(F + (long long)z * g.plane + (long long)y * g.pitch + x4);
-}
+// c1 (a - b) + c2 (c - d)
+__device__ __forceinline__ float d4f(float a, float b, float c, float d) { return kC1 * (a - b) + kC2 * (c - d); }
 
-__global__ void __launch_bounds__(128, 4) adj_v3_kernel(const AdjArgs3 A)
+// mu_p (the blocks of p3_kernel)
+__global__ void __launch_bounds__(128, 8) adj_p3_kernel(const AdjArgs3 A)
 {
     const Geo3 &g = A.g;
     const int x0 = 4 * (blockIdx.x * 32 + threadIdx.x);
     const int y = blockIdx.y * 4 + threadIdx.y;
     const int z = blockIdx.z;
-    if (x0 >= g.Nx || y >= g.Ny) return;
+    if (x0 >= g.Nx - 2 || y < 2 || y >= g.Ny - 2 || z < g.fs + 1 || z >= g.Nz - 2) return;
     const long long o = (long long)z * g.plane + (long long)y * g.pitch + x0;
-    // a2 times the mask of each velocity component at the neighbours the
-    // transposed gradient reads: x-1 .. x+1 (vx), rows y-2 .. y+1 (vy),
-    // planes z-2 .. z+1 (vz); the same for every shot
-    float mx[12], my[4][4], mz[4][4];
-    {
-        const float4 l = row4(g, A.a2, z, y, x0 - 4), c = row4(g, A.a2, z, y, x0), r = row4(g, A.a2, z, y, x0 + 4);
-        const float v[12] = {l.x, l.y, l.z, l.w, c.x, c.y, c.z, c.w, r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int i = 0; i < 12; ++i) mx[i] = in_vx(g, z, y, x0 - 4 + i) ? v[i] : 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float4 ay = row4(g, A.a2, z, y + k - 2, x0), az = row4(g, A.a2, z + k - 2, y, x0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            my[k][q] = in_vy(g, z, y + k - 2, x0 + q) ? f4(ay, q) : 0.f;
-            mz[k][q] = in_vz(g, z + k - 2, y, x0 + q) ? f4(az, q) : 0.f;
-        }
-    }
-    const float4 k2 = row4(g, A.k2, z, y, x0), k3 = row4(g, A.k3, z, y, x0), k4 = row4(g, A.k4, z, y, x0);
-    float g2[4] = {0.f, 0.f, 0.f, 0.f};
+    const float4 a1 = *reinterpret_cast<const float4 *>(A.a1 + o);
+    const float4 k1 = *reinterpret_cast<const float4 *>(A.k1 + o);
     for (int s = 0; s < g.n_shots; ++s) {
-        const float *L = A.lam_in + (long long)s * 4 * g.vol;
-        float *O = A.lam_out + (long long)s * 4 * g.vol;
-        const float *LX = L + g.vol, *LY = L + 2 * g.vol, *LZ = L + 3 * g.vol;
+        float *P = A.mu + (long long)s * 4 * g.vol;
+        const float *VX = P + g.vol, *VY = P + 2 * g.vol, *VZ = P + 3 * g.vol;
         if (s + 1 < g.n_shots) {
-            const float *N = L + 4 * g.vol + o;
+            const float *N = P + 4 * g.vol + o;
             prefetch_l2(N); prefetch_l2(N + g.vol); prefetch_l2(N + 2 * g.vol); prefetch_l2(N + 3 * g.vol);
-            if (A.G2) {
-                const long long js = (long long)g.n_shots * g.vol, jo = (long long)(s + 1) * g.vol + o;
-                prefetch_l2(A.img_j + jo); prefetch_l2(A.img_j + js + jo); prefetch_l2(A.img_j + 2 * js + jo);
-            }
         }
-        const float4 xl = row4(g, LX, z, y, x0 - 4), xc = row4(g, LX, z, y, x0), xr = row4(g, LX, z, y, x0 + 4);
-        const float lxs[12] = {xl.x, xl.y, xl.z, xl.w, xc.x, xc.y, xc.z, xc.w, xr.x, xr.y, xr.z, xr.w};
-        float4 ly[4], lz[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            ly[k] = row4(g, LY, z, y + k - 2, x0);
-            lz[k] = row4(g, LZ, z + k - 2, y, x0);
-        }
-        const float4 lp = *reinterpret_cast<const float4 *>(L + o);
-        float4 jx = make_float4(0.f, 0.f, 0.f, 0.f), jy = jx, jz = jx;
-        if (A.G2) {
-            const long long jo = (long long)s * g.vol + o, js = (long long)g.n_shots * g.vol;
-            jx = *reinterpret_cast<const float4 *>(A.img_j + jo);
-            jy = *reinterpret_cast<const float4 *>(A.img_j + js + jo);
-            jz = *reinterpret_cast<const float4 *>(A.img_j + 2 * js + jo);
-        }
-        float op[4], ox[4], oy[4], oz[4];
+        const float4 p = *reinterpret_cast<const float4 *>(P + o);
+        const float4 xl = ld4z(VX, o - 4, x0 >= 4), xc = ld4z(VX, o, true), xr = ld4z(VX, o + 4, x0 + 4 < g.pitch);
+        const float xs[12] = {xl.x, xl.y, xl.z, xl.w, xc.x, xc.y, xc.z, xc.w, xr.x, xr.y, xr.z, xr.w};
+        const float4 ym2 = ld4z(VY, o - 2 * g.pitch, true), ym1 = ld4z(VY, o - g.pitch, true), y0 = ld4z(VY, o, true),
+                     yp1 = ld4z(VY, o + g.pitch, true);
+        const float4 zm2 = ld4z(VZ, o - 2 * g.plane, z >= 2), zm1 = ld4z(VZ, o - g.plane, true), z0 = ld4z(VZ, o, true),
+                     zp1 = ld4z(VZ, o + g.plane, true);
+        float pv[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            // w = a2 lam on the component's mask; lp' = lp - sum_c G_c^T w
-            const float wx_m1 = mx[q + 3] * lxs[q + 3], wx_0 = mx[q + 4] * lxs[q + 4];
-            const float wx_m2 = mx[q + 2] * lxs[q + 2], wx_p1 = mx[q + 5] * lxs[q + 5];
-            const float wy_m2 = my[0][q] * f4(ly[0], q), wy_m1 = my[1][q] * f4(ly[1], q);
-            const float wy_0 = my[2][q] * f4(ly[2], q), wy_p1 = my[3][q] * f4(ly[3], q);
-            const float wz_m2 = mz[0][q] * f4(lz[0], q), wz_m1 = mz[1][q] * f4(lz[1], q);
-            const float wz_0 = mz[2][q] * f4(lz[2], q), wz_p1 = mz[3][q] * f4(lz[3], q);
-            const float gt = kC1 * (wx_m1 - wx_0) + kC2 * (wx_m2 - wx_p1) + kC1 * (wy_m1 - wy_0) +
-                             kC2 * (wy_m2 - wy_p1) + kC1 * (wz_m1 - wz_0) + kC2 * (wz_m2 - wz_p1);
-            op[q] = f4(lp, q) - gt;
+            float sum = d4f(xs[q + 4], xs[q + 3], xs[q + 5], xs[q + 2]) + d4f(f4(y0, q), f4(ym1, q), f4(yp1, q), f4(ym2, q)) +
+                        d4f(f4(z0, q), f4(zm1, q), f4(zp1, q), f4(zm2, q));
+            // the mirror plane's divergence, c2 mu_vz[fs], with the sign of p[fs-1] = -p[fs+1]
+            if (A.free_surface && z == g.fs + 1) sum -= kC2 * f4(zm1, q);
             const int x = x0 + q;
-            const float lxq = lxs[q + 4], lyq = f4(ly[2], q), lzq = f4(lz[2], q);
-            const bool bx = in_vx(g, z, y, x), by = in_vy(g, z, y, x), bz = in_vz(g, z, y, x);
-            ox[q] = bx ? (1.f - f4(k2, q)) * lxq : lxq;
-            oy[q] = by ? (1.f - f4(k3, q)) * lyq : lyq;
-            oz[q] = bz ? (1.f - f4(k4, q)) * lzq : lzq;
-            if (A.G2) {
-                if (bx) g2[q] -= lxq * f4(jx, q);
-                if (by) g2[q] -= lyq * f4(jy, q);
-                if (bz) g2[q] -= lzq * f4(jz, q);
-            }
+            pv[q] = x >= 2 && x < g.Nx - 2 ? (1.f - f4(k1, q)) * f4(p, q) + f4(a1, q) * sum : 0.f;
         }
-        *reinterpret_cast<float4 *>(O + o) = make_float4(op[0], op[1], op[2], op[3]);
-        *reinterpret_cast<float4 *>(O + g.vol + o) = make_float4(ox[0], ox[1], ox[2], ox[3]);
-        *reinterpret_cast<float4 *>(O + 2 * g.vol + o) = make_float4(oy[0], oy[1], oy[2], oy[3]);
-        *reinterpret_cast<float4 *>(O + 3 * g.vol + o) = make_float4(oz[0], oz[1], oz[2], oz[3]);
-    }
-    if (A.G2) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (x0 + q < g.Nx) neumaier3(A.G2[o + q], A.C2[o + q], g2[q]);
+        *reinterpret_cast<float4 *>(P + o) = make_float4(pv[0], pv[1], pv[2], pv[3]);
     }
 }
 
-__global__ void __launch_bounds__(128, 4) adj_p3_kernel(const AdjArgs3 A)
+// mu_vx, mu_vy, mu_vz and the gradient sums (one owner per cell)
+template <bool RHO>
+__global__ void __launch_bounds__(128, RHO ? 4 : 5) adj_v3_kernel(const AdjArgs3 A)
 {
     const Geo3 &g = A.g;
     const int x0 = 4 * (blockIdx.x * 32 + threadIdx.x);
     const int y = blockIdx.y * 4 + threadIdx.y;
     const int z = blockIdx.z;
-    if (x0 >= g.Nx || y >= g.Ny) return;
+    if (x0 >= g.Nx - 1 || y < 1 || y >= g.Ny - 1 || z < g.fs || z >= g.Nz - 1) return;
     const long long o = (long long)z * g.plane + (long long)y * g.pitch + x0;
-    // a1 times the p mask at the neighbours the transposed divergence reads:
-    // x-1 .. x+2, rows y-1 .. y+2, planes z-1 .. z+2 (the same for every shot)
-    float ux[12], uy[4][4], uz[4][4];
-    {
-        const float4 l = row4(g, A.a1, z, y, x0 - 4), c = row4(g, A.a1, z, y, x0), r = row4(g, A.a1, z, y, x0 + 4);
-        const float v[12] = {l.x, l.y, l.z, l.w, c.x, c.y, c.z, c.w, r.x, r.y, r.z, r.w};
-#pragma unroll
-        for (int i = 0; i < 12; ++i) ux[i] = in_p(g, z, y, x0 - 4 + i) ? v[i] : 0.f;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const float4 ay = row4(g, A.a1, z, y + k - 1, x0), az = row4(g, A.a1, z + k - 1, y, x0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            uy[k][q] = in_p(g, z, y + k - 1, x0 + q) ? f4(ay, q) : 0.f;
-            uz[k][q] = in_p(g, z + k - 1, y, x0 + q) ? f4(az, q) : 0.f;
-        }
-    }
-    const float4 k1 = row4(g, A.k1, z, y, x0);
-    float g1[4] = {0.f, 0.f, 0.f, 0.f};
+    const bool vy_row = y < g.Ny - 2, vz_row = z < g.Nz - 2;
+    const float4 a2 = *reinterpret_cast<const float4 *>(A.a2 + o), k2 = *reinterpret_cast<const float4 *>(A.k2 + o),
+                 k3 = *reinterpret_cast<const float4 *>(A.k3 + o), k4 = *reinterpret_cast<const float4 *>(A.k4 + o);
+    const bool p_row = z >= g.fs + 1 && z < g.Nz - 2 && y >= 2 && y < g.Ny - 2;
+    float g1[4] = {0.f, 0.f, 0.f, 0.f}, g2[4] = {0.f, 0.f, 0.f, 0.f};
     for (int s = 0; s < g.n_shots; ++s) {
-        const float *L = A.lam_in + (long long)s * 4 * g.vol;     // lp' and lam_c'
-        float *O = A.lam_out + (long long)s * 4 * g.vol;
+        const float *P = A.mu + (long long)s * 4 * g.vol;
+        float *VX = A.mu + ((long long)s * 4 + 1) * g.vol, *VY = VX + g.vol, *VZ = VY + g.vol;
+        const long long jo = (long long)s * g.vol + o, js = (long long)g.n_shots * g.vol;
         if (s + 1 < g.n_shots) {
-            const float *N = L + 4 * g.vol + o;
+            const float *N = P + 4 * g.vol + o;
             prefetch_l2(N); prefetch_l2(N + g.vol); prefetch_l2(N + 2 * g.vol); prefetch_l2(N + 3 * g.vol);
-            prefetch_l2(A.img_i + (long long)(s + 1) * g.vol + o);
+            prefetch_l2(A.img_i + jo + g.vol);
+            if (RHO) {
+                prefetch_l2(A.img_j + jo + g.vol); prefetch_l2(A.img_j + js + jo + g.vol);
+                prefetch_l2(A.img_j + 2 * js + jo + g.vol);
+            }
         }
-        const float4 pl = row4(g, L, z, y, x0 - 4), pc = row4(g, L, z, y, x0), pr = row4(g, L, z, y, x0 + 4);
+        const float4 pc = *reinterpret_cast<const float4 *>(P + o);
+        const float4 pl = ld4z(P, o - 4, x0 >= 4), pr = ld4z(P, o + 4, x0 + 4 < g.pitch);
         const float ps[12] = {pl.x, pl.y, pl.z, pl.w, pc.x, pc.y, pc.z, pc.w, pr.x, pr.y, pr.z, pr.w};
-        float4 py[4], pz[4];
+        const float4 ym1 = ld4z(P, o - g.pitch, true), yp1 = ld4z(P, o + g.pitch, true),
+                     yp2 = ld4z(P, o + 2 * g.pitch, vy_row);
+        const float4 zm1 = ld4z(P, o - g.plane, z >= 1), zp1 = ld4z(P, o + g.plane, true),
+                     zp2 = ld4z(P, o + 2 * g.plane, vz_row);
+        const float4 vx = *reinterpret_cast<const float4 *>(VX + o), vy = *reinterpret_cast<const float4 *>(VY + o),
+                     vz = *reinterpret_cast<const float4 *>(VZ + o);
+        if (p_row) {
+            const float4 im = *reinterpret_cast<const float4 *>(A.img_i + jo);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            py[k] = k == 1 ? pc : row4(g, L, z, y + k - 1, x0);
-            pz[k] = k == 1 ? pc : row4(g, L, z + k - 1, y, x0);
+            for (int q = 0; q < 4; ++q)
+                if (x0 + q >= 2 && x0 + q < g.Nx - 2) g1[q] += f4(pc, q) * f4(im, q);
         }
-        const float4 lvx = *reinterpret_cast<const float4 *>(L + g.vol + o);
-        const float4 lvy = *reinterpret_cast<const float4 *>(L + 2 * g.vol + o);
-        const float4 lvz = *reinterpret_cast<const float4 *>(L + 3 * g.vol + o);
-        const float4 im = *reinterpret_cast<const float4 *>(A.img_i + (long long)s * g.vol + o);
-        float op[4], ox[4], oy[4], oz[4];
+        if (RHO) {
+            // on the masks only: the imaging fields need not be written elsewhere
+            const float4 jx = *reinterpret_cast<const float4 *>(A.img_j + jo);
+            const float4 jy = ld4z(A.img_j, js + jo, vy_row), jz = ld4z(A.img_j, 2 * js + jo, vz_row);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int x = x0 + q;
+                if (x >= 1 && x < g.Nx - 2) g2[q] += f4(vx, q) * f4(jx, q);
+                if (x >= 1 && x < g.Nx - 1) g2[q] += f4(vy, q) * f4(jy, q) + f4(vz, q) * f4(jz, q);
+            }
+        }
+        float rx[4], ry[4], rz[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int x = x0 + q;
-            const float lp = ps[q + 4];
-            const bool mp = in_p(g, z, y, x);
-            op[q] = mp ? (1.f - f4(k1, q)) * lp : lp;
-            if (mp) g1[q] += lp * f4(im, q);
-            // u = a1 lp' on the p mask; lam_c = lam_c' - D_c^T u
-            const float u0 = ux[q + 4] * ps[q + 4], uxp1 = ux[q + 5] * ps[q + 5];
-            const float uxm1 = ux[q + 3] * ps[q + 3], uxp2 = ux[q + 6] * ps[q + 6];
-            ox[q] = f4(lvx, q) - (kC1 * (u0 - uxp1) + kC2 * (uxm1 - uxp2));
-            const float uym1 = uy[0][q] * f4(py[0], q), uyp1 = uy[2][q] * f4(py[2], q), uyp2 = uy[3][q] * f4(py[3], q);
-            oy[q] = f4(lvy, q) - (kC1 * (u0 - uyp1) + kC2 * (uym1 - uyp2));
-            const float uzm1 = uz[0][q] * f4(pz[0], q), uzp1 = uz[2][q] * f4(pz[2], q), uzp2 = uz[3][q] * f4(pz[3], q);
-            oz[q] = f4(lvz, q) - (kC1 * (u0 - uzp1) + kC2 * (uzm1 - uzp2));
+            const bool in = x >= 1 && x < g.Nx - 1;
+            const float dx = d4f(ps[q + 5], ps[q + 4], ps[q + 6], ps[q + 3]);
+            const float dy = d4f(f4(yp1, q), f4(pc, q), f4(yp2, q), f4(ym1, q));
+            float dz = d4f(f4(zp1, q), f4(pc, q), f4(zp2, q), f4(zm1, q));
+            // the p update read vz[fs-1] as vz[fs]: the mirror plane's gradient, c2 mu_p[fs+1]
+            if (A.free_surface && z == g.fs) dz += kC2 * f4(zp1, q);
+            rx[q] = in && x < g.Nx - 2 ? (1.f - f4(k2, q)) * f4(vx, q) + f4(a2, q) * dx : 0.f;
+            ry[q] = in && vy_row ? (1.f - f4(k3, q)) * f4(vy, q) + f4(a2, q) * dy : 0.f;
+            rz[q] = in && vz_row ? (1.f - f4(k4, q)) * f4(vz, q) + f4(a2, q) * dz : 0.f;
         }
-        *reinterpret_cast<float4 *>(O + o) = make_float4(op[0], op[1], op[2], op[3]);
-        *reinterpret_cast<float4 *>(O + g.vol + o) = make_float4(ox[0], ox[1], ox[2], ox[3]);
-        *reinterpret_cast<float4 *>(O + 2 * g.vol + o) = make_float4(oy[0], oy[1], oy[2], oy[3]);
-        *reinterpret_cast<float4 *>(O + 3 * g.vol + o) = make_float4(oz[0], oz[1], oz[2], oz[3]);
+        *reinterpret_cast<float4 *>(VX + o) = make_float4(rx[0], rx[1], rx[2], rx[3]);
+        *reinterpret_cast<float4 *>(VY + o) = make_float4(ry[0], ry[1], ry[2], ry[3]);
+        *reinterpret_cast<float4 *>(VZ + o) = make_float4(rz[0], rz[1], rz[2], rz[3]);
     }
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-        if (x0 + q < g.Nx) neumaier3(A.G1[o + q], A.C1[o + q], g1[q]);
+    auto add = [&](float *G, float *C, const float (&v)[4]) {
+        float4 s = *reinterpret_cast<float4 *>(G + o), c = *reinterpret_cast<float4 *>(C + o);
+        neumaier3(s.x, c.x, v[0]);
+        neumaier3(s.y, c.y, v[1]);
+        neumaier3(s.z, c.z, v[2]);
+        neumaier3(s.w, c.w, v[3]);
+        *reinterpret_cast<float4 *>(G + o) = s;
+        *reinterpret_cast<float4 *>(C + o) = c;
+    };
+    if (p_row) add(A.G1, A.C1, g1);
+    if (RHO) add(A.G2, A.C2, g2);
 }
 
-// dL/dwavelet[s, it] = dt * lam_p at the source cell, read after the adjoint
-// of the velocity updates and the free-surface fold (lam_p is then the
-// adjoint of p just after the source was added, acoustic_3d.py:153-163)
-__global__ void wavelet_grad3_kernel(const Geo3 g, const float *lam, const int *src, float *grad_wavelet, int it)
+// dL/dwavelet[s, it] = dt * lam_p at the source cell, after adj_p3 and the
+// pressure injection (lam_p is then the adjoint of p just after the source was
+// added, acoustic_3d.py:153-163).  The state keeps lam_p on the p mask only;
+// for a source off it, lam_p is the running sum of what reaches the cell: the
+// receivers in it and the divergence of mu_v, kept in off[s].  A source in
+// the mirror plane is overwritten by the mirror: zero.
+__global__ void wavelet_grad3_kernel(const AdjArgs3 A, const int *src, const int *rcv, const float *res_p,
+                                     float *grad_wavelet, float *off, int it)
 {
+    const Geo3 &g = A.g;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= g.n_shots) return;
-    const long long o = (long long)src[s] * g.plane + (long long)src[g.n_shots + s] * g.pitch + src[2 * g.n_shots + s];
-    grad_wavelet[(long long)s * g.nt + it] = g.dt * lam[(long long)s * 4 * g.vol + o];
+    const int z = src[s], y = src[g.n_shots + s], x = src[2 * g.n_shots + s];
+    const long long o = (long long)z * g.plane + (long long)y * g.pitch + x;
+    const float *P = A.mu + (long long)s * 4 * g.vol;
+    float lam;
+    if (in_p(g, z, y, x)) {
+        lam = P[o] / A.a1[o];
+    } else if (A.free_surface && z == g.fs - 1) {
+        lam = 0.f;
+    } else {
+        auto at = [&](int f, int zz, int yy, int xx) {
+            return zz < 0 || zz >= g.Nz || yy < 0 || yy >= g.Ny || xx < 0 || xx >= g.Nx
+                       ? 0.f
+                       : P[(long long)f * g.vol + (long long)zz * g.plane + (long long)yy * g.pitch + xx];
+        };
+        lam = off[s];
+        if (res_p)
+            for (int r = 0; r < g.n_rcv; ++r)
+                if (rcv[r] == z && rcv[g.n_rcv + r] == y && rcv[2 * g.n_rcv + r] == x)
+                    lam += res_p[((long long)s * g.nt + it) * g.n_rcv + r];
+        lam += d4f(at(1, z, y, x), at(1, z, y, x - 1), at(1, z, y, x + 1), at(1, z, y, x - 2)) +
+               d4f(at(2, z, y, x), at(2, z, y - 1, x), at(2, z, y + 1, x), at(2, z, y - 2, x)) +
+               d4f(at(3, z, y, x), at(3, z - 1, y, x), at(3, z + 1, y, x), at(3, z - 2, y, x));
+        off[s] = lam;
+    }
+    grad_wavelet[(long long)s * g.nt + it] = g.dt * lam;
 }
 
-// Adjoint of the recording: lam[field][receiver cell] += res[field][s][it][r]
-__global__ void inj3_kernel(const Geo3 g, float *lam, const int *rcv, const float *res_p, const float *res_vx,
-                            const float *res_vy, const float *res_vz, int it)
+// Adjoint of the recording: mu_f[receiver cell] += coefficient * res_f[s][it][r]
+// on the mask of field f; a receiver in the mirror plane fs - 1 recorded
+// -p[fs+1] and vz[fs].  pressure: p, else the velocities.
+__global__ void inj3_kernel(const AdjArgs3 A, const int *rcv, const float *res_p, const float *res_vx,
+                            const float *res_vy, const float *res_vz, int pressure, int it)
 {
+    const Geo3 &g = A.g;
     const long long n = (long long)g.n_shots * g.n_rcv;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const int s = (int)(i / g.n_rcv), r = (int)(i % g.n_rcv);
-        const long long o = (long long)rcv[r] * g.plane + (long long)rcv[g.n_rcv + r] * g.pitch + rcv[2 * g.n_rcv + r];
-        float *L = lam + (long long)s * 4 * g.vol;
+        const int z = rcv[r], y = rcv[g.n_rcv + r], x = rcv[2 * g.n_rcv + r];
+        const bool mir = A.free_surface && z == g.fs - 1;
+        const long long row = (long long)y * g.pitch + x, o = (long long)z * g.plane + row;
+        float *M = A.mu + (long long)s * 4 * g.vol;
         const long long t = ((long long)s * g.nt + it) * g.n_rcv + r;
-        if (res_p) atomicAdd(L + o, res_p[t]);     // receivers may share a cell
-        if (res_vx) atomicAdd(L + g.vol + o, res_vx[t]);
-        if (res_vy) atomicAdd(L + 2 * g.vol + o, res_vy[t]);
-        if (res_vz) atomicAdd(L + 3 * g.vol + o, res_vz[t]);
+        // receivers may share a cell
+        if (pressure) {
+            const int zp = mir ? g.fs + 1 : z;
+            const long long op = (long long)zp * g.plane + row;
+            if (in_p(g, zp, y, x)) atomicAdd(M + op, mir ? -A.a1[op] * res_p[t] : A.a1[op] * res_p[t]);
+            continue;
+        }
+        if (res_vx && in_vx(g, z, y, x)) atomicAdd(M + g.vol + o, A.a2[o] * res_vx[t]);
+        if (res_vy && in_vy(g, z, y, x)) atomicAdd(M + 2 * g.vol + o, A.a2[o] * res_vy[t]);
+        const int zv = mir ? g.fs : z;
+        const long long ov = (long long)zv * g.plane + row;
+        if (res_vz && in_vz(g, zv, y, x)) atomicAdd(M + 3 * g.vol + ov, A.a2[ov] * res_vz[t]);
     }
 }
 
-// Free-surface folds of the adjoint: field f, plane fs - 1 folded into plane
-// fs - 1 + to with sign, then cleared (the adjoints of vz[fs-1] = vz[fs]
-// and p[fs-1] = -p[fs+1]).
-__global__ void fold3_kernel(const Geo3 g, float *lam, int field, int to, float sign)
-{
-    const long long n = (long long)g.n_shots * g.plane;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const long long s = i / g.plane, r = i % g.plane;
-        float *F = lam + (s * 4 + field) * g.vol;
-        F[(long long)(g.fs - 1 + to) * g.plane + r] += sign * F[(long long)(g.fs - 1) * g.plane + r];
-        F[(long long)(g.fs - 1) * g.plane + r] = 0.f;
-    }
-}
-
-// dL/dvp, dL/drho on the unpadded grid: the chain rule through a1 = rho c^2
-// dt / dz and a2 = dt / (rho dz) on the padded grid, summed over the padded
+// dL/dvp, dL/drho on the unpadded grid: G1 = sum mu_p I and G2 = sum mu_v J
+// are a1 dL/da1 and -a2 dL/da2, so with a1 = rho c^2 dt / dz and a2 = dt /
+// (rho dz) dL/dc = 2 G1 / c and dL/drho = (G1 + G2) / rho, summed over the padded
 // cells each model cell was replicated into (the adjoint of pad_model_3d).  A
 // cell on an edge or a corner of the model collects pml^2 or pml^3 of them: a
 // warp shares those (one thread per corner took 0.67 ms at 18 layers).
-__global__ void grad3_finish_kernel(const Geo3 g, const float *vp, const float *rho, float dz, const float *G1,
+__global__ void grad3_finish_kernel(const Geo3 g, const float *vp, const float *rho, const float *G1,
                                     const float *C1, const float *G2, const float *C2, float *grad_vp,
                                     float *grad_rho)
 {
@@ -608,9 +588,8 @@ __global__ void grad3_finish_kernel(const Geo3 g, const float *vp, const float *
         len = (idx == n_in - 1 ? n_in + 2 * g.pml - 1 : idx + g.pml) - lo + 1;
     };
     auto write = [&](long long i, double s1, double s2) {
-        const double c = vp[i], den = rho[i], dt = g.dt;
-        grad_vp[i] = (float)(s1 * 2.0 * den * c * dt / dz);
-        if (grad_rho) grad_rho[i] = (float)(s1 * c * c * dt / dz - s2 * dt / (den * den * dz));
+        grad_vp[i] = (float)(2.0 * s1 / (double)vp[i]);
+        if (grad_rho) grad_rho[i] = (float)((s1 + s2) / (double)rho[i]);
     };
     auto edge = [&](int idx, int n_in) { return idx == 0 || idx == n_in - 1 ? 1 : 0; };
     const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x, threads = (long long)gridDim.x * blockDim.x;

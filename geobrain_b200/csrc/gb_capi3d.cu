@@ -368,7 +368,7 @@ int gb3_forward(const gb3_model_desc *desc, const int64_t *src_x, const int64_t 
 namespace {
 
 struct Layout3B {
-    size_t err, state, state2, coef, src, rcv, lam_a, lam_b, img_i, img_j, g1, c1, g2, c2, total;
+    size_t err, state, state2, coef, src, rcv, off, mu, img_i, img_j, g1, c1, g2, c2, total;
 };
 
 Layout3B layout3b(const Geo3 &g, int K, bool rho, int mode)
@@ -382,8 +382,8 @@ Layout3B layout3b(const Geo3 &g, int K, bool rho, int mode)
     L.coef = o; o = align256(o + 6 * (size_t)g.vol * 4);
     L.src = o; o = align256(o + 3 * (size_t)g.n_shots * 4);
     L.rcv = o; o = align256(o + 3 * (size_t)std::max(g.n_rcv, 1) * 4);
-    L.lam_a = o; o = align256(o + st);
-    L.lam_b = o; o = align256(o + st);
+    L.off = o; o = align256(o + (size_t)g.n_shots * 4);
+    L.mu = o; o = align256(o + st);
     L.img_i = o; o = align256(o + (size_t)K * f);
     L.img_j = o; o = align256(o + (rho ? 3 * (size_t)K * f : 0));
     L.g1 = o; o = align256(o + (size_t)g.vol * 4);
@@ -441,7 +441,7 @@ int gb3_backward(const gb3_model_desc *desc, const int64_t *src_x, const int64_t
     int *d_err = reinterpret_cast<int *>(ws + L.err);
     float *coef = reinterpret_cast<float *>(ws + L.coef);
     int *d_src = reinterpret_cast<int *>(ws + L.src), *d_rcv = reinterpret_cast<int *>(ws + L.rcv);
-    float *lam_a = reinterpret_cast<float *>(ws + L.lam_a), *lam_b = reinterpret_cast<float *>(ws + L.lam_b);
+    float *mu = reinterpret_cast<float *>(ws + L.mu), *off = reinterpret_cast<float *>(ws + L.off);
     float *img_i = reinterpret_cast<float *>(ws + L.img_i), *img_j = reinterpret_cast<float *>(ws + L.img_j);
     float *G1 = reinterpret_cast<float *>(ws + L.g1), *C1 = reinterpret_cast<float *>(ws + L.c1);
     float *G2 = with_rho ? reinterpret_cast<float *>(ws + L.g2) : nullptr;
@@ -452,8 +452,8 @@ int gb3_backward(const gb3_model_desc *desc, const int64_t *src_x, const int64_t
     // columns [Nx, pitch) of both state buffers stay zero: a checkpoint brings them in as zeros
     if (fused) GB_CUDA(cudaMemsetAsync(state2, 0, state_bytes, st));
     GB_CUDA(cudaMemsetAsync(coef, 0, 6 * (size_t)g.vol * 4, st));
-    GB_CUDA(cudaMemsetAsync(lam_a, 0, state_bytes, st));
-    GB_CUDA(cudaMemsetAsync(lam_b, 0, state_bytes, st));
+    GB_CUDA(cudaMemsetAsync(mu, 0, state_bytes, st));
+    GB_CUDA(cudaMemsetAsync(off, 0, (size_t)g.n_shots * 4, st));
     GB_CUDA(cudaMemsetAsync(G1, 0, (size_t)g.vol * 4, st));
     GB_CUDA(cudaMemsetAsync(C1, 0, (size_t)g.vol * 4, st));
     if (with_rho) {
@@ -475,7 +475,9 @@ int gb3_backward(const gb3_model_desc *desc, const int64_t *src_x, const int64_t
     A.g = g;
     A.a1 = F.a1; A.k1 = F.k1; A.a2 = F.a2; A.k2 = F.k2; A.k3 = F.k3; A.k4 = F.k4;
     A.G1 = G1; A.C1 = C1; A.G2 = G2; A.C2 = C2;
+    A.mu = mu;
     const bool fs = desc->free_surface != 0;
+    A.free_surface = fs;
     Fused3 FU{};
     Fused3Args FA{};
     if (fused) {
@@ -508,10 +510,7 @@ int gb3_backward(const gb3_model_desc *desc, const int64_t *src_x, const int64_t
         }
         // adjoint steps, last to first
         for (int it = t1 - 1; it >= t0; --it) {
-            if (g.n_rcv > 0 && (res_p || res_vx || res_vy || res_vz))
-                inj3_kernel<<<(g.n_shots * g.n_rcv + 255) / 256, 256, 0, st>>>(g, lam_a, d_rcv, res_p, res_vx,
-                                                                              res_vy, res_vz, it);
-            if (fs) fold3_kernel<<<148, 256, 0, st>>>(g, lam_a, 3, 1, 1.f);
+            const int nb = (g.n_shots * g.n_rcv + 255) / 256;
             if (imaging) {
                 A.img_i = imaging + (size_t)it * blk;
                 A.img_j = with_rho ? imaging + (size_t)it * blk + field : nullptr;
@@ -519,19 +518,19 @@ int gb3_backward(const gb3_model_desc *desc, const int64_t *src_x, const int64_t
                 A.img_i = img_i + (size_t)(it - t0) * field;
                 A.img_j = with_rho ? img_j + (size_t)(it - t0) * 3 * field : nullptr;
             }
-            A.lam_in = lam_a;
-            A.lam_out = lam_b;
-            adj_v3_kernel<<<grid, block, 0, st>>>(A);
-            if (fs) fold3_kernel<<<148, 256, 0, st>>>(g, lam_b, 0, 2, -1.f);
-            if (grad_wavelet)
-                wavelet_grad3_kernel<<<(g.n_shots + 127) / 128, 128, 0, st>>>(g, lam_b, d_src, grad_wavelet, it);
-            A.lam_in = lam_b;
-            A.lam_out = lam_a;
+            if (g.n_rcv > 0 && (res_vx || res_vy || res_vz))
+                inj3_kernel<<<nb, 256, 0, st>>>(A, d_rcv, res_p, res_vx, res_vy, res_vz, 0, it);
             adj_p3_kernel<<<grid, block, 0, st>>>(A);
+            if (g.n_rcv > 0 && res_p) inj3_kernel<<<nb, 256, 0, st>>>(A, d_rcv, res_p, res_vx, res_vy, res_vz, 1, it);
+            if (grad_wavelet)
+                wavelet_grad3_kernel<<<(g.n_shots + 127) / 128, 128, 0, st>>>(A, d_src, d_rcv, g.n_rcv > 0 ? res_p : nullptr,
+                                                                              grad_wavelet, off, it);
+            if (with_rho) adj_v3_kernel<true><<<grid, block, 0, st>>>(A);
+            else adj_v3_kernel<false><<<grid, block, 0, st>>>(A);
             GB_CUDA(cudaGetLastError());
         }
     }
-    grad3_finish_kernel<<<4 * 148, 256, 0, st>>>(g, vp, rho, desc->dz, G1, C1, G2, C2, grad_vp, grad_rho);
+    grad3_finish_kernel<<<4 * 148, 256, 0, st>>>(g, vp, rho, G1, C1, G2, C2, grad_vp, grad_rho);
     GB_CUDA(cudaGetLastError());
     return GB_OK;
 }

@@ -340,3 +340,38 @@ def test_cuda_3d_fused_step_at_the_benchmark_size(cuda_device, mode):
     for k in KEYS:
         np.testing.assert_array_equal(fused[k], split[k], err_msg=k)
     assert np.abs(fused["p"]).max() > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("free_surface", [False, True])
+def test_cuda_3d_gradients_at_the_rims(cuda_device, free_surface):
+    """The scaled in-place adjoint where its masks, mirror planes and scaling
+    end: a source off the pressure mask (its wavelet gradient is a running
+    sum), receivers in the padded border, in one cell twice, in a source's
+    cell and in the mirror plane under a free surface, a ragged grid.  dL/dvp,
+    dL/drho and dL/dsrc_v against the float64 oracle, 1e-4 as the tests above."""
+    from geobrain_b200.wave import acoustic_forward_kernel_3d, bc_pml_3d
+    rng = np.random.default_rng(17)
+    nz, ny, nx, nabc, nt = 17, 14, 39, 6, 48
+    vp = (2000 + 800 * rng.random((nz, ny, nx))).astype(np.float32)
+    rho = (1900 + 300 * rng.random((nz, ny, nx))).astype(np.float32)
+    damp = bc_pml_3d(nx, ny, nz, 10.0, 10.0, 10.0, nabc, float(vp.max()), free_surface=False).astype(np.float32)
+    w = rng.standard_normal((4, nt)).astype(np.float32)
+    top = 0 if free_surface else -nabc
+    src = dict(src_x=np.array([4, 30, -nabc, nx + nabc - 1]), src_y=np.array([2, 9, 5, 7]),
+               src_z=np.array([1, 11, 8, top]), src_v=w)
+    rcv = dict(rcv_x=np.array([0, 10, 10, -nabc, 30, nx + nabc - 2]), rcv_y=np.array([1, 5, 5, 5, 9, 3]),
+               rcv_z=np.array([0, 3, 3, 8, -1, nz + nabc - 2]))
+    kw = dict(nz=nz, ny=ny, nx=nx, nt=nt, dt=1e-3, nabc=nabc, free_surface=free_surface, **rcv)
+    res = {k: rng.standard_normal((4, nt, 6)).astype(np.float32) for k in ("p", "vx", "vy", "vz")}
+    t = lambda a: torch.as_tensor(a, device=cuda_device)
+    v, r, s = (t(a).requires_grad_(True) for a in (vp, rho, w))
+    out = acoustic_forward_kernel_3d(dx=10.0, dy=10.0, dz=10.0, src_n=4, rcv_n=6, damp=t(damp), vp=v, rho=r,
+                                     device=cuda_device, **kw, **dict(src, src_v=s))
+    sum((t(res[k]) * out[k]).sum() for k in res).backward()
+    gv, gr, gw = o3.gradient(dz=10.0, damp=damp, vp=vp, rho=rho, with_wavelet=True, **kw, **src,
+                             **{f"res_{k}": x for k, x in res.items()})
+    assert orc.rel_l2(v.grad.cpu().numpy(), gv) < 1e-4
+    assert orc.rel_l2(r.grad.cpu().numpy(), gr) < 1e-4
+    for i in range(4):
+        assert orc.rel_l2(s.grad[i].cpu().numpy(), gw[i]) < 1e-4, i
