@@ -110,6 +110,7 @@ def _forward(prep: _Prepared, vps, rhos, want_energy: bool, stores=None):
 class _BatchFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, prep, opts, *params):
+        ctx.set_materialize_grads(False)     # a trace the loss does not use has no adjoint source
         n = len(prep.plans)
         vps = [p.detach().to(torch.float32).contiguous() for p in params[:n]]
         rhos = [p.detach().to(torch.float32).contiguous() for p in params[n:]]

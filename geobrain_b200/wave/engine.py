@@ -407,6 +407,7 @@ class AcousticFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, vp, rho, plan, damp, src_v, opts):
         dev = vp.device
+        ctx.set_materialize_grads(False)     # a trace the loss does not use has no adjoint source
         src_v = src_v.detach().contiguous()
         vp32 = vp.detach().to(torch.float32).contiguous()
         rho32 = rho.detach().to(torch.float32).contiguous()

@@ -102,6 +102,7 @@ class _Function3D(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, vp, rho, wavelet, run, K, imaging_cache):
+        ctx.set_materialize_grads(False)     # a trace the loss does not use has no adjoint source
         # the C calls read run.w, the wavelet this graph node differentiates
         run.w = wavelet.detach().contiguous()
         vp32 = vp.detach().to(torch.float32).contiguous()
