@@ -21,6 +21,19 @@
 // Cells outside the update masks never depend on the model, so their adjoint
 // is dropped (held at zero); that keeps every stencil read mask-free.
 // dL/dvp and dL/drho follow from G1, G2 in grad_finish_kernel.
+//
+// CPML layers (the forward's psi' = b psi + a g on every derivative g) need
+// the adjoints eta of the four memory variables.  With b = 1 + a the step's
+// transpose is the one above with the stencils taken over
+//   e = bh mu_v - ah eta_v   (stage A),   f = b mu_p - a eta_p   (stage B),
+// x and z each with their own profile and eta, no damping, and
+//   eta_v <- bh (eta_v - mu_v),   eta_p <- b (eta_p - mu_p)
+// in place of theirs (mu before the update of its stage B).  Where a profile
+// vanishes (a = 0, b = 1; most of the grid) e and f are mu and eta is never
+// read: tiles clear of the layers take the fast path, and the others load eta
+// only in the rows and columns of a layer.  (As gather kernels over all cells,
+// 11 state planes a shot and 12 coefficient planes, the adjoint took 140 us a
+// step at 460 x 1260 with 8 shots.)
 #pragma once
 
 #include "gb_fwd.cuh"
@@ -54,7 +67,48 @@ struct AdjArgs {
     float *img_base;
     long long img_step;
     int img_t0;
+    // CPML: the forward's profiles, and eta [S][px, pz, vx, vz][plane] read
+    // and written (two levels, as the state)
+    const float *cpml;
+    const float *eta_in;
+    float *eta_out;
 };
+
+// b v - a eta at 4 cells (b = 1, a = 0 outside a layer: v itself).
+__device__ __forceinline__ float4 cpml_mix(const float4 &v, const float4 &b, const float4 &a, const float4 &h)
+{
+    return make_float4(b.x * v.x - a.x * h.x, b.y * v.y - a.y * h.y, b.z * v.z - a.z * h.z, b.w * v.w - a.w * h.w);
+}
+__device__ __forceinline__ float4 splat4(float v) { return make_float4(v, v, v, v); }
+// eta <- b (eta - mu) at 4 cells of a layer
+__device__ __forceinline__ void cpml_eta(bool on, const float4 &mu, const float4 &b, const float4 &h, float *out)
+{
+    if (on) stg4(out, make_float4(b.x * (h.x - mu.x), b.y * (h.y - mu.y), b.z * (h.z - mu.z), b.w * (h.w - mu.w)));
+}
+// v <- b v - a eta on N rows of a z window from tile row `row` on (rows z0 - 2R
+// + row + t), cells (x, x + 3) of lane columns, in batches so that the loads
+// of a batch are in flight together
+template <int N, int R, int TZ>
+__device__ __forceinline__ void cpml_mix_rows(float4 (&v)[N], int n, int row, const CpmlTile<R, TZ> &cp, int half,
+                                              const float *eta, int z0, int gx0, const StepGeom &g)
+{
+    constexpr int B = 5;
+    const bool cols = gx0 >= 0 && gx0 < g.pitch;
+#pragma unroll
+    for (int t0 = 0; t0 < N; t0 += B) {
+        float4 h[B];
+#pragma unroll
+        for (int i = 0; i < B && t0 + i < N; ++i) {
+            const int r = row + t0 + i;
+            h[i] = ldg4_if(t0 + i < n && cols && cp.az[half][min(r, Geo<R, TZ>::ZR - 1)] != 0.f,
+                           eta + (long long)(z0 - 2 * R + r) * g.pitch + gx0);
+        }
+#pragma unroll
+        for (int i = 0; i < B && t0 + i < N; ++i)
+            if (t0 + i < n)
+                v[t0 + i] = cpml_mix(v[t0 + i], splat4(cp.bz[half][row + t0 + i]), splat4(cp.az[half][row + t0 + i]), h[i]);
+    }
+}
 
 __device__ __forceinline__ void neumaier_add(float &s, float &c, float x)
 {
@@ -68,7 +122,7 @@ __device__ __forceinline__ void neumaier_add(float &s, float &c, float x)
 
 // IMGF: storage format of the imaging fields (kImg*), or -1 to read it from
 // A.img_fmt at run time (batched launches, where it varies per model).
-template <int R, int TZ, bool FS, bool RHO, int IMGF>
+template <int R, int TZ, bool FS, bool RHO, int IMGF, bool CPML = false>
 __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMap *mVX, const CUtensorMap *mVZ,
                                          const CUtensorMap *mA1, const CUtensorMap *mA2,
                                          const AdjArgs &__restrict__ A, const int group, const int tile)
@@ -107,6 +161,8 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
     const bool fast = A.tile_fast[tile] != 0;
     const int rcv0 = A.rcv_ptr[tile], rcv1 = A.rcv_ptr[tile + 1];
     const bool has_rcv = rcv1 > rcv0 && (A.res_p || A.res_vx || A.res_vz);
+    __shared__ std::conditional_t<CPML, CpmlTile<R, TZ>, CpmlNone> cp;
+    if (CPML && !fast) cp.load(A.cpml, g, z0, x0);
     __syncthreads();
     if (threadIdx.x == 0) {
         mbar_arrive_expect_tx(&bars[2], SM::COEF_BYTES);
@@ -140,6 +196,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
     for (int k = 0; k < ns; ++k) {
         const int s = s0 + k;
         const int b = k & 1;
+        const float *const eta_in = CPML ? A.eta_in + (long long)s * 4 * g.plane : nullptr;
         // imaging fields of this shot's tile cells: issued now, used in stage B
         ImgRaw im[G::LV], jx[G::LV], jz[G::LV];
 #pragma unroll
@@ -201,6 +258,11 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
 #pragma unroll
             for (int t = 0; t < G::LP + 2 * R - 1; ++t)
                 wz[t] = (t < rc + 2 * R - 1) ? lds4(sVZ + (rb + t) * RW + 4 * lane) : zero4();
+            if constexpr (CPML) {
+                // e_z on the window's rows
+                if (!fast)
+                    cpml_mix_rows<G::LP + 2 * R - 1, R, TZ>(wz, rc + 2 * R - 1, rb, cp, 1, eta_in + 3 * g.plane, z0, gx0, g);
+            }
 #pragma unroll
             for (int u = 0; u < G::LP; ++u) {
                 if (u < rc) {
@@ -216,7 +278,22 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                     } else {
                         const bool row_in = gz >= g.p_r0 && gz <= g.p_r1;
                         if (row_in && (gx0 + 3 >= g.p_c0) && (gx0 <= g.p_c1)) {
-                            divergence4<R>(sVX + r * VXW, lane, wz, u, g.c, D);
+                            if constexpr (CPML) {
+                                float4 e[3], h[3];
+#pragma unroll
+                                for (int t = 0; t < 3; ++t) {
+                                    const int gx = gx0 - 4 + 4 * t;
+                                    h[t] = ldg4_if(gx >= 0 && gx < g.pitch && any4(lds4(cp.ax[1] + 4 * lane + 4 * t)),
+                                                   eta_in + 2 * g.plane + (long long)gz * g.pitch + gx);
+                                }
+#pragma unroll
+                                for (int t = 0; t < 3; ++t)
+                                    e[t] = cpml_mix(lds4(sVX + r * VXW + 4 * lane + 4 * t), lds4(cp.bx[1] + 4 * lane + 4 * t),
+                                                    lds4(cp.ax[1] + 4 * lane + 4 * t), h[t]);
+                                divergence4_of<R>(e[0], e[1], e[2], wz, u, g.c, D);
+                            } else {
+                                divergence4<R>(sVX + r * VXW, lane, wz, u, g.c, D);
+                            }
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
                                 float d = D[q];
@@ -259,6 +336,12 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
 #pragma unroll
             for (int t = 0; t < G::LV + 2 * R - 1; ++t)
                 wp[t] = (t < vcnt + 2 * R - 1) ? lds4(sP + (vb + 1 + t) * RW + 4 * lane) : zero4();
+            if constexpr (CPML) {
+                // f_z on the window's rows
+                if (!fast)
+                    cpml_mix_rows<G::LV + 2 * R - 1, R, TZ>(wp, vcnt + 2 * R - 1, vb + 1 + R, cp, 0, eta_in + g.plane, z0,
+                                                            gx0, g);
+            }
 #pragma unroll
             for (int u = 0; u < G::LV; ++u) {
                 if (u < vcnt) {
@@ -267,8 +350,28 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                     const int gz = z0 + rv;
                     if (fast || (gz < g.Nz && gx0 < g.Nx)) {
                         float Dx[4], Dz[4];
-                        const float4 mp1 = wp[u + R - 1];       // mu_p row rr
-                        grad_x4<R>(sP + rr * RW, lane, g.c, Dx, mp1);
+                        // mu_p row rr
+                        const float4 mp1 = CPML && !fast ? lds4(sP + rr * RW + 4 * lane) : wp[u + R - 1];
+                        if constexpr (CPML) {
+                            if (!fast) {
+                                float4 f[3], h[3];
+#pragma unroll
+                                for (int t = 0; t < 3; ++t) {
+                                    const int gx = gx0 - 4 + 4 * t;
+                                    h[t] = ldg4_if(gx >= 0 && gx < g.pitch && any4(lds4(cp.ax[0] + 4 * lane + 4 * t)),
+                                                   eta_in + (long long)gz * g.pitch + gx);
+                                }
+#pragma unroll
+                                for (int t = 0; t < 3; ++t)
+                                    f[t] = cpml_mix(lds4(sP + rr * RW + 4 * lane - 4 + 4 * t),
+                                                    lds4(cp.bx[0] + 4 * lane + 4 * t), lds4(cp.ax[0] + 4 * lane + 4 * t), h[t]);
+                                grad_x4_of<R>(f[0], f[1], f[2], g.c, Dx);
+                            } else {
+                                grad_x4<R>(sP + rr * RW, lane, g.c, Dx, mp1);
+                            }
+                        } else {
+                            grad_x4<R>(sP + rr * RW, lane, g.c, Dx, mp1);
+                        }
                         grad_z4<R>(wp, u, g.c, Dz);
                         const float4 vx1 = lds4(sVX + rr * VXW + 4 * lane + 4);
                         const float4 vz1 = lds4(sVZ + (rv + 2 * R) * RW + 4 * lane);
@@ -301,9 +404,22 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                             const bool any_v = (vx_row && gx0 + 3 >= g.vx_c0 && gx0 <= g.vx_c1) ||
                                                (vz_row && gx0 + 3 >= g.vz_c0 && gx0 <= g.vz_c1);
                             const bool any_p = p_row && gx0 + 3 >= g.p_c0 && gx0 <= g.p_c1;
+                            if constexpr (CPML) {
+                                float *eo = A.eta_out + (long long)s * 4 * g.plane + o;
+                                const float *ei = eta_in + o;
+                                const bool lx = any4(lds4(cp.ax[0] + 4 * lane + 4)), lxh = any4(lds4(cp.ax[1] + 4 * lane + 4));
+                                const bool lz = cp.az[0][rv + 2 * R] != 0.f, lzh = cp.az[1][rv + 2 * R] != 0.f;
+                                const float4 h0 = ldg4_if(lx, ei), h1 = ldg4_if(lz, ei + g.plane),
+                                             h2 = ldg4_if(lxh, ei + 2 * g.plane), h3 = ldg4_if(lzh, ei + 3 * g.plane);
+                                cpml_eta(lx, mp1, lds4(cp.bx[0] + 4 * lane + 4), h0, eo);
+                                cpml_eta(lz, mp1, splat4(cp.bz[0][rv + 2 * R]), h1, eo + g.plane);
+                                cpml_eta(lxh, vx1, lds4(cp.bx[1] + 4 * lane + 4), h2, eo + 2 * g.plane);
+                                cpml_eta(lzh, vz1, splat4(cp.bz[1][rv + 2 * R]), h3, eo + 3 * g.plane);
+                            }
                             if (any_v) {
-                                const float4 k2 = ldg4(A.k2 + o);
-                                const float4 k3 = ldg4(A.k3 + o);
+                                // no damping with CPML
+                                const float4 k2 = CPML ? zero4() : ldg4(A.k2 + o);
+                                const float4 k3 = CPML ? zero4() : ldg4(A.k3 + o);
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
                                     const int gx = gx0 + q;
@@ -324,7 +440,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                                 }
                             }
                             if (any_p) {
-                                const float4 k1 = ldg4(A.k1 + o);
+                                const float4 k1 = CPML ? zero4() : ldg4(A.k1 + o);
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
                                     const int gx = gx0 + q;
@@ -374,7 +490,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
     }
 }
 
-template <int R, int TZ, bool FS, bool RHO, int IMGF>
+template <int R, int TZ, bool FS, bool RHO, int IMGF, bool CPML = false>
 __global__ void __launch_bounds__(NTHR, TZ <= 16 ? 2 : 1)
 adj_step_kernel(const __grid_constant__ CUtensorMap mP, const __grid_constant__ CUtensorMap mVX,
                 const __grid_constant__ CUtensorMap mVZ, const __grid_constant__ CUtensorMap mA1,
@@ -383,7 +499,7 @@ adj_step_kernel(const __grid_constant__ CUtensorMap mP, const __grid_constant__ 
     const int group = A.grp0 + (int)(blockIdx.x % A.grp_count);
     const int rank = (int)(blockIdx.x / A.grp_count);
     const int tile = A.tile_order ? A.tile_order[rank] : rank;
-    adj_body<R, TZ, FS, RHO, IMGF>(&mP, &mVX, &mVZ, &mA1, &mA2, A, group, tile);
+    adj_body<R, TZ, FS, RHO, IMGF, CPML>(&mP, &mVX, &mVZ, &mA1, &mA2, A, group, tile);
 }
 
 template <int R, int TZ>

@@ -10,7 +10,6 @@
 #include "gb_misfit.cuh"
 #include "gb_stream.cuh"
 #include "gb_fwd.cuh"
-#include "gb_cpml_adj.cuh"
 #include "gb_resident.cuh"
 
 #include <cudaTypedefs.h>
@@ -440,7 +439,7 @@ struct Layout {
     size_t err, coef, fields, energy, src, rcv_ptr, rcv_ent, tile_fast, sched, amax, cpml, psi, total;
     size_t res_ptr, res_ent, res_x;           // resident forward: receiver CSR, exchange strips
     // gradient only
-    size_t mu, img, g1, c1, g2, c2, arcv_ptr, arcv_ent, cprcv, cpcoef;
+    size_t mu, eta, img, g1, c1, g2, c2, arcv_ptr, arcv_ent;
     int n_img;
 };
 
@@ -486,8 +485,8 @@ Layout layout(const gb_plan *p, int with_gradient = 0, int checkpoint_every = 0,
     if (with_gradient > 0) {
         const size_t K = std::max(1, std::min(checkpoint_every, p->d.nt));
         const size_t G = p->n_groups;
-        // adjoint state: p, vx, vz (and, with CPML, the four memory variables)
-        L.mu = o; o = align256(o + S * (p->cpml ? kCpmlPlanes : 2 * 3) * p->plane * 4);
+        L.mu = o; o = align256(o + S * 2 * 3 * p->plane * 4);
+        if (p->cpml) L.eta = o, o = align256(o + S * 2 * 4 * p->plane * 4);   // adjoints of the memory variables
         L.img = o; o = align256(o + K * L.n_img * S * p->plane * img_esize(img_fmt));
         L.g1 = o; o = align256(o + G * p->plane * 4);
         L.c1 = o; o = align256(o + G * p->plane * 4);
@@ -497,10 +496,6 @@ Layout layout(const gb_plan *p, int with_gradient = 0, int checkpoint_every = 0,
         }
         L.arcv_ptr = o; o = align256(o + (p->n_tiles + 1) * 4);
         L.arcv_ent = o; o = align256(o + std::max<size_t>(p->arcv_ent.size(), 1) * 16);
-        if (p->cpml) {
-            L.cprcv = o; o = align256(o + std::max<size_t>(p->d.n_rcv, 1) * 8);
-            L.cpcoef = o; o = align256(o + (size_t)kCpmlCoefPlanes * p->plane * 4);
-        }
     }
     L.total = o;
     return L;
@@ -508,8 +503,9 @@ Layout layout(const gb_plan *p, int with_gradient = 0, int checkpoint_every = 0,
 
 // The plan's forward step kernel: the streaming one when the plan asks for it
 // (no free surface, 16-row tiles), else the tile kernel.
-StepKernel fwd_kernel(int R, int tz, bool fs, bool en, int im)
+StepKernel fwd_kernel(int R, int tz, bool fs, bool en, int im, bool cpml)
 {
+    if (cpml) return R == 2 ? fwd_cpml_kernel_r2(tz, fs, en, im) : fwd_cpml_kernel_r4(tz, fs, en, im);
     if (R == 2) return fwd_tile_kernel_r2(tz, fs, en, im);
     if (R == 4) return fwd_tile_kernel_r4(tz, fs, en, im);
     return StepKernel{};
@@ -518,11 +514,12 @@ StepKernel fwd_kernel(int R, int tz, bool fs, bool en, int im)
 StepKernel fwd_kernel_for(const gb_plan *P, bool en, int im)
 {
     if (P->stream_usable()) return fwd_stream_kernel_for(P->R, en, im);
-    return fwd_kernel(P->R, P->tz, P->d.free_surface != 0, en, im);
+    return fwd_kernel(P->R, P->tz, P->d.free_surface != 0, en, im, P->cpml);
 }
 
-StepKernel adj_kernel(int R, int tz, bool fs, bool rho, int img_fmt)
+StepKernel adj_kernel(int R, int tz, bool fs, bool rho, int img_fmt, bool cpml)
 {
+    if (cpml) return R == 2 ? adj_cpml_kernel_r2(tz, fs, rho, img_fmt) : adj_cpml_kernel_r4(tz, fs, rho, img_fmt);
     if (R == 2) return adj_tile_kernel_r2(tz, fs, rho, img_fmt);
     if (R == 4) return adj_tile_kernel_r4(tz, fs, rho, img_fmt);
     return StepKernel{};
@@ -562,10 +559,12 @@ int make_maps(const gb_plan *P, const float *buf, const float *a1, const float *
 }
 
 // Per-tile fast-path flags (needs the coefficient planes).
+// rows, cols: how far past the p rectangle the CPML profiles must vanish too.
 int launch_tile_flags(gb_plan *P, const StepGeom &g, const float *k1, const float *k2, const float *k3, int *flags,
-                      cudaStream_t st)
+                      cudaStream_t st, int rows = 0, int cols = 0)
 {
-    const int4 still = P->cpml ? P->cpml_still : int4{-(1 << 24), 1 << 24, -(1 << 24), 1 << 24};
+    int4 still{-(1 << 24), 1 << 24, -(1 << 24), 1 << 24};
+    if (P->cpml) still = int4{P->cpml_still.x + rows, P->cpml_still.y - rows, P->cpml_still.z + cols, P->cpml_still.w - cols};
     if (P->R == 2 && P->tz == 16) tile_fast_kernel<2, 16><<<P->n_tiles, 256, 0, st>>>(g, k1, k2, k3, flags, still);
     if (P->R == 2 && P->tz == 32) tile_fast_kernel<2, 32><<<P->n_tiles, 256, 0, st>>>(g, k1, k2, k3, flags, still);
     if (P->R == 4 && P->tz == 16) tile_fast_kernel<4, 16><<<P->n_tiles, 256, 0, st>>>(g, k1, k2, k3, flags, still);
@@ -1131,105 +1130,6 @@ int forward_resident(gb_plan *P, const Layout &L, char *ws, const Setup &Su, flo
             it0 = it1;
         }
     }
-    return GB_OK;
-}
-
-// Gradient of a CPML plan: the adjoint sweep of gb_cpml_adj.cuh over every
-// step, from imaging fields the forward kept for all nt steps (no recompute,
-// so no memory variables need checkpointing).
-int backward_cpml(gb_plan *P, const float *vp, const float *rho, const float *damp, const float *res_p,
-                  const float *res_vx, const float *res_vz, const gb_grad_store *store, float *grad_vp,
-                  float *grad_rho, float *grad_wavelet, void *workspace, size_t workspace_bytes, cudaStream_t st)
-{
-    const gb_model_desc &d = P->d;
-    if (store->cached_steps < d.nt)
-        return fail(GB_E_UNSUPPORTED, "CPML gradients need every step's imaging fields in the store (cached_steps = nt)");
-    const bool rho_fields = store->with_rho != 0;
-    const int ifmt = store->imaging_format;
-    const Layout L = layout(P, rho_fields ? 2 : 1, 1, ifmt);
-    char *ws = aligned_ws(workspace);
-    if (!workspace || workspace_bytes < L.total + (size_t)(ws - reinterpret_cast<char *>(workspace)))
-        return fail(GB_E_WORKSPACE, "workspace too small");
-    Setup Su;
-    if (int rc = common_setup(P, L, ws, vp, rho, damp, st, &Su)) return rc;
-    const int S = d.n_shots;
-    float *lam = reinterpret_cast<float *>(ws + L.mu);   // [S][kCpmlPlanes][plane]
-    float *G1 = reinterpret_cast<float *>(ws + L.g1), *C1 = reinterpret_cast<float *>(ws + L.c1);
-    float *G2 = rho_fields ? reinterpret_cast<float *>(ws + L.g2) : nullptr;
-    float *C2 = rho_fields ? reinterpret_cast<float *>(ws + L.c2) : nullptr;
-    GB_CUDA(cudaMemsetAsync(lam, 0, (size_t)S * kCpmlPlanes * P->plane * 4, st));
-    GB_CUDA(cudaMemsetAsync(G1, 0, (size_t)P->n_groups * P->plane * 4, st));
-    GB_CUDA(cudaMemsetAsync(C1, 0, (size_t)P->n_groups * P->plane * 4, st));
-    if (G2) {
-        GB_CUDA(cudaMemsetAsync(G2, 0, (size_t)P->n_groups * P->plane * 4, st));
-        GB_CUDA(cudaMemsetAsync(C2, 0, (size_t)P->n_groups * P->plane * 4, st));
-    }
-    int2 *d_rcv = reinterpret_cast<int2 *>(ws + L.cprcv);
-    std::vector<int2> hr(d.n_rcv);
-    for (int r = 0; r < d.n_rcv; ++r) hr[r] = make_int2(P->rcv_z[r], P->rcv_x[r]);
-    // pageable host vector: cudaMemcpyAsync copies it before returning
-    if (d.n_rcv) GB_CUDA(cudaMemcpyAsync(d_rcv, hr.data(), hr.size() * 8, cudaMemcpyHostToDevice, st));
-
-    const StepGeom g = P->geom();
-    float *cpcoef = reinterpret_cast<float *>(ws + L.cpcoef);
-    cpml_adj_coef_kernel<<<4 * 148, 256, 0, st>>>(g, Su.a1, Su.a2, Su.cpml, cpcoef);
-    ++P->launches;
-    CpmlAdjArgs4 A{};
-    A.g = g;
-    A.a1 = Su.a1;
-    A.a2 = Su.a2;
-    A.cp = cpcoef;
-    A.lam = lam;
-    A.img_field_stride = (long long)S * P->plane;
-    A.img_fmt = ifmt;
-    A.G1 = G1; A.C1 = C1; A.G2 = G2; A.C2 = C2;
-    const bool fs = d.free_surface != 0;
-    A.free_surface = fs;
-    const bool inject = d.n_rcv > 0 && (res_p || res_vx || res_vz);
-    const size_t step_img = (size_t)(rho_fields ? 3 : 1) * S * P->plane;
-    const dim3 block(32, 4), grid((P->Nx + 127) / 128, (P->Nz + 4 * kCpLZ - 1) / (4 * kCpLZ), P->n_groups);
-    const int fold_blocks = (int)std::min<long long>(1024, ((long long)S * P->Nx + 255) / 256);
-    P->mark(2, true, st);
-    P->phase_steps[2] += d.nt;
-    int sv = 0, sp = 0;   // the memory-variable slots read this step
-    for (int it = d.nt - 1; it >= 0; --it) {
-        if (inject) {
-            cpml_inject_kernel<<<std::max(1, std::min(1024, (S * d.n_rcv + 255) / 256)), 256, 0, st>>>(
-                g, lam, d_rcv, res_p, res_vx, res_vz, it);
-            ++P->launches;
-        }
-        if (fs) {
-            cpml_fold_kernel<<<fold_blocks, 256, 0, st>>>(g, lam, kLamVZ, 1, 1.f);
-            ++P->launches;
-        }
-        A.img = img_at(store->imaging, (size_t)it * step_img, img_esize(ifmt));
-        A.psi_in = kPsiV0 + 2 * sv;
-        A.psi_out = kPsiV0 + 2 * (sv ^ 1);
-        if (P->R == 4) cpml_adj_v_kernel<4><<<grid, block, 0, st>>>(A);
-        else cpml_adj_v_kernel<2><<<grid, block, 0, st>>>(A);
-        sv ^= 1;
-        if (fs) {
-            cpml_fold_kernel<<<fold_blocks, 256, 0, st>>>(g, lam, kLamP, 2, -1.f);
-            ++P->launches;
-        }
-        if (grad_wavelet) {
-            cpml_wavelet_grad_kernel<<<(S + 127) / 128, 128, 0, st>>>(g, lam, Su.d_src, Su.d_src + S, grad_wavelet,
-                                                                       it);
-            ++P->launches;
-        }
-        A.psi_in = kPsiP0 + 2 * sp;
-        A.psi_out = kPsiP0 + 2 * (sp ^ 1);
-        if (P->R == 4) cpml_adj_p_kernel<4><<<grid, block, 0, st>>>(A);
-        else cpml_adj_p_kernel<2><<<grid, block, 0, st>>>(A);
-        sp ^= 1;
-        P->launches += 2;
-        GB_CUDA(cudaGetLastError());
-    }
-    P->mark(2, false, st);
-    grad_finish_kernel<<<4 * 148, 256, 0, st>>>(vp, rho, G1, C1, G2, C2, P->n_groups, P->plane, d.nz, d.nx, d.nabc,
-                                                P->pitch, grad_vp, grad_rho);
-    GB_CUDA(cudaGetLastError());
-    ++P->launches;
     return GB_OK;
 }
 
@@ -1885,9 +1785,9 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
         GB_CUDA(cudaMemsetAsync(grad_wavelet, 0, (size_t)P->d.n_shots * P->d.nt * 4,
                                 reinterpret_cast<cudaStream_t>(stream)));
     }
-    if (P->cpml)
-        return backward_cpml(P, vp, rho, damp, res_p, res_vx, res_vz, store, grad_vp, grad_rho, grad_wavelet,
-                             workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
+    // the memory variables have no checkpoints: the CPML adjoint recomputes nothing
+    if (P->cpml && store->cached_steps < P->d.nt)
+        return fail(GB_E_UNSUPPORTED, "CPML gradients need every step's imaging fields in the store (cached_steps = nt)");
     const gb_model_desc &d = P->d;
     const int S = d.n_shots;
     const int K = std::min<int>(store->checkpoint_every, d.nt);
@@ -1924,10 +1824,21 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
         GB_CUDA(cudaMemsetAsync(C2, 0, (size_t)P->n_groups * P->plane * 4, st));
     }
 
+    float *eta[2] = {nullptr, nullptr};
+    if (P->cpml) {
+        const size_t n = (size_t)S * 4 * P->plane;
+        eta[0] = reinterpret_cast<float *>(ws + L.eta);
+        eta[1] = eta[0] + n;
+        GB_CUDA(cudaMemsetAsync(eta[0], 0, 2 * n * 4, st));
+        // the adjoint's stage A mixes eta into the velocities of the whole
+        // stage: its fast tiles keep R more rows and 4 more columns off the layers
+        if (int rc = launch_tile_flags(P, P->geom(), Su.k1, Su.k2, Su.k3, Su.tile_fast, st, P->R, 4)) return rc;
+    }
+
     const bool fs = d.free_surface != 0;
     const StepKernel KF = fwd_kernel_for(P, false, rho_fields ? 2 : 1);
     // cached and recomputed imaging fields share the store's format
-    const StepKernel KA = adj_kernel(P->R, P->tz, fs, rho_fields, ifmt);
+    const StepKernel KA = adj_kernel(P->R, P->tz, fs, rho_fields, ifmt, P->cpml);
     if (int rc = prepare_kernel(KF)) return rc;
     if (int rc = prepare_kernel(KA)) return rc;
     Maps fmaps[2], amaps[2];
@@ -1959,6 +1870,7 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
     A.grad_wavelet = grad_wavelet;
     A.src_z = Su.d_src;
     A.src_x = Su.d_src + S;
+    A.cpml = Su.cpml;
 
     GroupStreams gs;
     if (int rc = group_streams(P, st, &gs)) return rc;
@@ -1979,6 +1891,8 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
         auto one_step = [&](int it) -> int {
             A.it = it;
             A.out = mu[cur ^ 1];
+            A.eta_in = eta[cur];
+            A.eta_out = eta[cur ^ 1];
             A.img = img_at(img_base, (size_t)(it - t0) * step_img, img_esize(img_fmt));
             A.img_fmt = img_fmt;
             for (int i = 0; i < gs.n; ++i) {
@@ -2013,6 +1927,8 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
                         AdjArgs Bj = B;
                         Bj.it = j;
                         Bj.out = mu[(j & 1) ^ 1];
+                        Bj.eta_in = eta[j & 1];
+                        Bj.eta_out = eta[(j & 1) ^ 1];
                         for (int i = 0; i < g.n; ++i) {
                             int g0, gc;
                             launch_groups(g, i, P->n_groups, &g0, &gc);

@@ -23,6 +23,8 @@
 
 #include "gb_stencil.cuh"
 
+#include <type_traits>
+
 namespace gb {
 
 struct StepGeom {
@@ -109,12 +111,49 @@ __device__ __forceinline__ bool tile_is_interior(const StepGeom &g, int z0, int 
            x0 + TX - 1 <= g.vz_c1;
 }
 
+// The CPML profiles around one tile, in shared memory: b and a at integer and
+// half rows z0 - 2R .. z0 + TZ + 2R - 1, and at integer and half columns
+// x0 - 8 .. x0 + 127; b = 1, a = 0 off the grid.  Where a is zero a memory
+// variable stays zero and is neither read nor written.
+template <int R, int TZ>
+struct CpmlTile {
+    float bz[2][Geo<R, TZ>::ZR], az[2][Geo<R, TZ>::ZR];   // [0] integer, [1] half
+    alignas(16) float bx[2][VXW];
+    alignas(16) float ax[2][VXW];
+
+    __device__ __forceinline__ void load(const float *prof, const StepGeom &g, int z0, int x0)
+    {
+        for (int i = threadIdx.x; i < Geo<R, TZ>::ZR; i += NTHR) {
+            const int z = z0 - 2 * R + i;
+            const bool in = z >= 0 && z < g.Nz;
+            for (int h = 0; h < 2; ++h) {
+                bz[h][i] = in ? prof[2 * h * g.Nz + z] : 1.f;
+                az[h][i] = in ? prof[(2 * h + 1) * g.Nz + z] : 0.f;
+            }
+        }
+        const float *xp = prof + 4 * g.Nz;
+        for (int i = threadIdx.x; i < VXW; i += NTHR) {
+            const int x = x0 - 8 + i;
+            const bool in = x >= 0 && x < g.Nx;
+            for (int h = 0; h < 2; ++h) {
+                bx[h][i] = in ? xp[2 * h * g.pitch + x] : 1.f;
+                ax[h][i] = in ? xp[(2 * h + 1) * g.pitch + x] : 0.f;
+            }
+        }
+    }
+};
+struct CpmlNone {
+    __device__ __forceinline__ void load(const float *, const StepGeom &, int, int) {}
+};
+__device__ __forceinline__ bool any4(const float4 &a) { return a.x != 0.f || a.y != 0.f || a.z != 0.f || a.w != 0.f; }
+__device__ __forceinline__ float4 ldg4_if(bool on, const float *p) { return on ? ldg4(p) : zero4(); }
+
 // IMG: 0 no imaging fields; 1 store I = -div(v^n) on the p mask (velocity
 // gradient); 2 also store Jx = dx(p), Jz = dz(p) on the vx / vz masks (density).
 // The body of one CTA: shots [s0, s0 + ns) (ns <= kMaxShotsPerCta) of tile
 // `tile` of the model A describes; the maps are the TMA descriptors of the
 // input state and of the a1 / a2 planes.
-template <int R, int TZ, bool FS, bool ENERGY, int IMG>
+template <int R, int TZ, bool FS, bool ENERGY, int IMG, bool CPML = false>
 __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMap *mVX, const CUtensorMap *mVZ,
                                          const CUtensorMap *mA1, const CUtensorMap *mA2,
                                          const FwdArgs &__restrict__ A, const int tile, const int s0, const int ns)
@@ -161,6 +200,8 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
     const bool fast = A.tile_fast[tile] != 0;
     const int rcv0 = A.rcv_ptr[tile], rcv1 = A.rcv_ptr[tile + 1];
     const bool has_rcv = rcv1 > rcv0 && (A.tr_p || A.tr_vx || A.tr_vz);
+    __shared__ std::conditional_t<CPML, CpmlTile<R, TZ>, CpmlNone> cp;
+    if (CPML && !fast) cp.load(A.cpml, g, z0, x0);
     if (!__syncthreads_and(mbar_wait_bounded(&bars[2], 0))) {
         if (threadIdx.x == 0) {
             atomicExch(A.err, -4);
@@ -230,15 +271,15 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                         if (row_in && (gx0 + 3 >= g.p_c0) && (gx0 <= g.p_c1)) {
                             const long long o = (long long)gz * g.pitch + gx0;
                             float4 img;
-                            if (A.cpml) {
+                            if constexpr (CPML) {
                                 // psi' = b psi + a d, p' = p - a1 ((Dx + psi_x') + (Dz + psi_z'))
+                                const float bz = cp.bz[0][r + R], az = cp.az[0][r + R];
+                                const float4 bx = lds4(cp.bx[0] + 4 * lane + 4), ax = lds4(cp.ax[0] + 4 * lane + 4);
+                                const bool lx = any4(ax), lz = az != 0.f;
+                                const long long po = (long long)s * 4 * g.plane + o;
+                                const float4 ox = ldg4_if(lx, A.psi_in + po), oz = ldg4_if(lz, A.psi_in + po + g.plane);
                                 float Dx[4], Dz[4];
                                 divergence4_split<R>(sVX + r * VXW, lane, wz, u, g.c, Dx, Dz);
-                                const float bz = A.cpml[gz], az = A.cpml[g.Nz + gz];
-                                const float *xp = A.cpml + 4 * g.Nz;
-                                const float4 bx = ldg4(xp + gx0), ax = ldg4(xp + g.pitch + gx0);
-                                const long long po = (long long)s * 4 * g.plane + o;
-                                const float4 ox = ldg4(A.psi_in + po), oz = ldg4(A.psi_in + po + g.plane);
                                 float4 nx = ox, nz = oz;
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
@@ -253,8 +294,8 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                                         at(img, q) = -sd;
                                     }
                                 }
-                                stg4(A.psi_out + po, nx);
-                                stg4(A.psi_out + po + g.plane, nz);
+                                if (lx) stg4(A.psi_out + po, nx);
+                                if (lz) stg4(A.psi_out + po + g.plane, nz);
                             } else {
                                 divergence4<R>(sVX + r * VXW, lane, wz, u, g.c, D);
                                 const float4 k1 = ldg4(A.k1 + o);
@@ -336,13 +377,14 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                             const bool vz_row = gz >= g.vz_r0 && gz <= g.vz_r1;
                             const bool need = (vx_row && gx0 + 3 >= g.vx_c0 && gx0 <= g.vx_c1) ||
                                               (vz_row && gx0 + 3 >= g.vz_c0 && gx0 <= g.vz_c1);
-                            if (need && A.cpml) {
+                            if constexpr (CPML) {
                                 // psi' = b psi + a G, v' = v - a2 (G + psi')
-                                const float bz = A.cpml[2 * g.Nz + gz], az = A.cpml[3 * g.Nz + gz];
-                                const float *xp = A.cpml + 4 * g.Nz;
-                                const float4 bx = ldg4(xp + 2 * g.pitch + gx0), ax = ldg4(xp + 3 * g.pitch + gx0);
+                                const float bz = cp.bz[1][rv + 2 * R], az = cp.az[1][rv + 2 * R];
+                                const float4 bx = lds4(cp.bx[1] + 4 * lane + 4), ax = lds4(cp.ax[1] + 4 * lane + 4);
+                                const bool lx = need && any4(ax), lz = need && az != 0.f;
                                 const long long po = (long long)s * 4 * g.plane + o;
-                                const float4 ox = ldg4(A.psi_in + po + 2 * g.plane), oz = ldg4(A.psi_in + po + 3 * g.plane);
+                                const float4 ox = ldg4_if(lx, A.psi_in + po + 2 * g.plane),
+                                             oz = ldg4_if(lz, A.psi_in + po + 3 * g.plane);
                                 float4 nx = ox, nz = oz;
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
@@ -358,8 +400,8 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                                         at(vz, q) = __fsub_rn(at(vz, q), __fmul_rn(at(a2, q), at(jz, q)));
                                     }
                                 }
-                                stg4(A.psi_out + po + 2 * g.plane, nx);
-                                stg4(A.psi_out + po + 3 * g.plane, nz);
+                                if (lx) stg4(A.psi_out + po + 2 * g.plane, nx);
+                                if (lz) stg4(A.psi_out + po + 3 * g.plane, nz);
                             } else if (need) {
                                 const float4 k2 = ldg4(A.k2 + o);
                                 const float4 k3 = ldg4(A.k3 + o);
@@ -443,7 +485,7 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
 // Single-model launch: blockIdx covers shot groups [grp0, grp0 + grp_count)
 // of every tile (one launch for all groups, or one per group when the groups
 // run on their own streams), in the order of the work list when there is one.
-template <int R, int TZ, bool FS, bool ENERGY, int IMG>
+template <int R, int TZ, bool FS, bool ENERGY, int IMG, bool CPML = false>
 __global__ void __launch_bounds__(NTHR, TZ <= 16 ? 2 : 1)
 fwd_step_kernel(const __grid_constant__ CUtensorMap mP, const __grid_constant__ CUtensorMap mVX,
                 const __grid_constant__ CUtensorMap mVZ, const __grid_constant__ CUtensorMap mA1,
@@ -461,7 +503,7 @@ fwd_step_kernel(const __grid_constant__ CUtensorMap mP, const __grid_constant__ 
         s0 = group * A.g.shots_per_cta;
         ns = min(A.g.n_shots - s0, A.g.shots_per_cta);
     }
-    fwd_body<R, TZ, FS, ENERGY, IMG>(&mP, &mVX, &mVZ, &mA1, &mA2, A, tile, s0, ns);
+    fwd_body<R, TZ, FS, ENERGY, IMG, CPML>(&mP, &mVX, &mVZ, &mA1, &mA2, A, tile, s0, ns);
 }
 
 template <int R, int TZ>

@@ -19,11 +19,17 @@ struct StepKernel {
 // unsupported combination.  gb_pick_fwd2.cu / gb_pick_fwd4.cu.
 StepKernel fwd_tile_kernel_r2(int tz, bool fs, bool en, int img);
 StepKernel fwd_tile_kernel_r4(int tz, bool fs, bool en, int img);
+// the same with CPML layers.  gb_pick_cpml_fwd2.cu / gb_pick_cpml_fwd4.cu.
+StepKernel fwd_cpml_kernel_r2(int tz, bool fs, bool en, int img);
+StepKernel fwd_cpml_kernel_r4(int tz, bool fs, bool en, int img);
 // fwd_stream_kernel<R, ENERGY, IMG> (gb_stream.cuh).  gb_pick_stream.cu.
 StepKernel fwd_stream_kernel_for(int R, bool en, int img);
 // adj_step_kernel<R, TZ, FS, RHO, IMGF> (gb_adj.cuh).  gb_pick_adj2.cu / gb_pick_adj4.cu.
 StepKernel adj_tile_kernel_r2(int tz, bool fs, bool rho, int img_fmt);
 StepKernel adj_tile_kernel_r4(int tz, bool fs, bool rho, int img_fmt);
+// adj_step_kernel with CPML layers.  gb_pick_cpml_adj2.cu / gb_pick_cpml_adj4.cu.
+StepKernel adj_cpml_kernel_r2(int tz, bool fs, bool rho, int img_fmt);
+StepKernel adj_cpml_kernel_r4(int tz, bool fs, bool rho, int img_fmt);
 // fwd_batch_kernel / adj_batch_kernel (gb_batch.cuh), 16-row tiles.  gb_pick_batch.cu.
 StepKernel fwd_batch_kernel_for(int R, bool fs, bool en, int img);
 // imgf: the imaging format all models of the batch store, or -1 (per model)

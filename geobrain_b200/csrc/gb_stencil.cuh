@@ -15,15 +15,13 @@ namespace gb {
 // vxr: the row of the vx rectangle (136 wide, column 0 = x0 - 8); the lane's
 // first column j = x0 - 4 + 4*lane sits at vxr[4*lane + 4].  wz: window of
 // vz rows with wz[u + R] = row i.
+// divergence4_of takes the lane's three vx quads.
 template <int R>
-__device__ __forceinline__ void divergence4(const float *vxr, int lane, const float4 *wz, int u,
-                                            const float (&c)[4], float (&D)[4])
+__device__ __forceinline__ void divergence4_of(const float4 &e0, const float4 &e1, const float4 &e2, const float4 *wz,
+                                               int u, const float (&c)[4], float (&D)[4])
 {
     float e[12];
     {
-        const float4 e0 = lds4(vxr + 4 * lane);
-        const float4 e1 = lds4(vxr + 4 * lane + 4);
-        const float4 e2 = lds4(vxr + 4 * lane + 8);
         e[0] = e0.x; e[1] = e0.y; e[2] = e0.z; e[3] = e0.w;
         e[4] = e1.x; e[5] = e1.y; e[6] = e1.z; e[7] = e1.w;
         e[8] = e2.x; e[9] = e2.y; e[10] = e2.z; e[11] = e2.w;
@@ -36,6 +34,12 @@ __device__ __forceinline__ void divergence4(const float *vxr, int lane, const fl
             d = __fmaf_rn(c[k], ((e[q + 4 + k] - e[q + 3 - k]) + at(wz[u + R + k], q)) - at(wz[u + R - 1 - k], q), d);
         D[q] = d;
     }
+}
+template <int R>
+__device__ __forceinline__ void divergence4(const float *vxr, int lane, const float4 *wz, int u,
+                                            const float (&c)[4], float (&D)[4])
+{
+    divergence4_of<R>(lds4(vxr + 4 * lane), lds4(vxr + 4 * lane + 4), lds4(vxr + 4 * lane + 8), wz, u, c, D);
 }
 
 // The two parts of divergence4 kept apart (the CPML option needs each one):
@@ -72,12 +76,11 @@ __device__ __forceinline__ void divergence4_split(const float *vxr, int lane, co
 // first column j sits at pr[4*lane] and its own cells are f1 (the callers'
 // z-windows hold them).
 template <int R>
-__device__ __forceinline__ void grad_x4(const float *pr, int lane, const float (&c)[4], float (&D)[4], const float4 &f1)
+__device__ __forceinline__ void grad_x4_of(const float4 &f0, const float4 &f1, const float4 &f2, const float (&c)[4],
+                                           float (&D)[4])
 {
     float f[12];
     {
-        const float4 f0 = lds4(pr + 4 * lane - 4);
-        const float4 f2 = lds4(pr + 4 * lane + 4);
         f[0] = f0.x; f[1] = f0.y; f[2] = f0.z; f[3] = f0.w;
         f[4] = f1.x; f[5] = f1.y; f[6] = f1.z; f[7] = f1.w;
         f[8] = f2.x; f[9] = f2.y; f[10] = f2.z; f[11] = f2.w;
@@ -89,6 +92,11 @@ __device__ __forceinline__ void grad_x4(const float *pr, int lane, const float (
         for (int k = 0; k < R; ++k) d = __fmaf_rn(c[k], f[q + 5 + k] - f[q + 4 - k], d);
         D[q] = d;
     }
+}
+template <int R>
+__device__ __forceinline__ void grad_x4(const float *pr, int lane, const float (&c)[4], float (&D)[4], const float4 &f1)
+{
+    grad_x4_of<R>(lds4(pr + 4 * lane - 4), f1, lds4(pr + 4 * lane + 4), c, D);
 }
 
 // z-derivative of p at the staggered vz points:
