@@ -132,6 +132,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
     using SM = StepSmem<R, TZ>;
     const StepGeom &__restrict__ g = A.g;
     extern __shared__ __align__(128) float smem[];
+    __shared__ unsigned s_done;   // warps that have finished a shot, over all shots
     float *sA1 = smem + 2 * G::STAGE_FL;
     float *sA2 = sA1 + SM::A1_FL;
     uint64_t *bars = reinterpret_cast<uint64_t *>(sA1 + SM::COEF_FL);
@@ -147,6 +148,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
         mbar_init(&bars[1], 1);
         mbar_init(&bars[2], 1);
         fence_mbar_init();
+        s_done = 0;
     }
     grid_dependency_wait();
     grid_launch_dependents();
@@ -211,9 +213,8 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
             }
         }
         // every thread waits (bounded) for this shot's stage; no CTA barrier
-        // here: the refill of shot k-1's buffer waits for the mid-shot
-        // barrier below, which every thread reaches only after finishing
-        // shot k-1.  A give-up sets the status word and the launch runs on
+        // here: shot k-1's buffer is refilled by the last warp to finish that
+        // shot.  A give-up sets the status word and the launch runs on
         // (every thread still meets every barrier); its results are void.
         if (!mbar_wait_bounded(&bars[b], (k >> 1) & 1)) atomicExch(A.err, -4);
         float *sP = smem + b * G::STAGE_FL;
@@ -316,11 +317,6 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
             }
         }
         __syncthreads();
-        // every thread is done with shot k-1: refill its buffer with shot k+1
-        // (its generic-proxy writes were fenced at the end of shot k-1)
-        if (threadIdx.x == 0 && k >= 1 && k + 1 < ns)
-            stage_loads<R>(mP, mVX, mVZ, smem + (b ^ 1) * G::STAGE_FL, &bars[b ^ 1], G::STAGE_BYTES, x0, z0,
-                           s + 1, G::P_FL, G::VX_FL);
         if (A.grad_wavelet && threadIdx.x == 0) {
             // the tile that owns the source cell: mu_p / a1 there is lambda_p
             const int sz = A.src_z[s], sx = A.src_x[s];
@@ -459,9 +455,8 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                 }
             }
         }
-        // order this shot's generic-proxy shared-memory writes before the TMA
-        // that refills the buffer (after the next shot's mid-shot barrier)
-        fence_proxy_async_smem();
+        if (k + 2 < ns && last_warp_of_shot(&s_done, lane))
+            stage_loads<R>(mP, mVX, mVZ, sP, &bars[b], G::STAGE_BYTES, x0, z0, s + 2, G::P_FL, G::VX_FL);
     }
 
     // compensated accumulation of this step's partial sums into the group's

@@ -87,6 +87,27 @@ __device__ __forceinline__ void stage_loads(const CUtensorMap *mP, const CUtenso
     tma_load_3d(buf + P_FL + VX_FL, mVZ, bar, x0 - 4, z0 - 2 * R, 3 * s + 2);
 }
 
+// Called by whole warps at the end of a shot: true in one lane of the last of
+// the CTA's warps to come.  That lane refills the shot's buffer at once: its
+// own and the other warps' accesses are ordered before the TMA writes by the
+// proxy fence of every thread and the counter.  No warp comes for shot k + 1
+// before all have come for shot k (the barrier in the middle of a shot), so
+// one counter does.
+// (A refill by thread 0 after the next shot's middle barrier left a load half
+// a shot's time, about 1.5 us, to arrive.)
+__device__ __forceinline__ bool last_warp_of_shot(unsigned *done, int lane)
+{
+    static_assert((NWARP & (NWARP - 1)) == 0, "the counter's low bits count one shot's warps");
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane != 0) return false;
+    unsigned n;
+    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(n) : "r"(smem_u32(done)) : "memory");
+    if ((n & (NWARP - 1)) != NWARP - 1) return false;
+    fence_proxy_async_smem();
+    return true;
+}
+
 // Shared-memory layout of both step kernels: two field stages, then a1 on
 // the p rectangle and a2 on the tile rows (loaded once per CTA), then the
 // mbarriers.
@@ -163,6 +184,7 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
     const StepGeom &__restrict__ g = A.g;
     extern __shared__ __align__(128) float smem[];
     __shared__ int2 s_src[kMaxShotsPerCta];   // (z, x) source cell of each shot of this CTA
+    __shared__ unsigned s_done;               // warps that have finished a shot, over all shots
     float *sA1 = smem + 2 * G::STAGE_FL;
     float *sA2 = sA1 + SM::A1_FL;
     uint64_t *bars = reinterpret_cast<uint64_t *>(sA1 + SM::COEF_FL);
@@ -176,6 +198,7 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
         mbar_init(&bars[1], 1);
         mbar_init(&bars[2], 1);
         fence_mbar_init();
+        s_done = 0;
     }
     grid_dependency_wait();
     grid_launch_dependents();
@@ -225,9 +248,8 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
         const int s = s0 + k;
         const int b = k & 1;
         // every thread waits (bounded) for this shot's stage; no CTA barrier
-        // here: the refill of shot k-1's buffer waits for the mid-shot
-        // barrier below, which every thread reaches only after finishing
-        // shot k-1.  A give-up sets the status word and the launch runs on
+        // here: shot k-1's buffer is refilled by the last warp to finish that
+        // shot.  A give-up sets the status word and the launch runs on
         // (every thread still meets every barrier); its results are void.
         if (!mbar_wait_bounded(&bars[b], (k >> 1) & 1)) atomicExch(A.err, -4);
         float *sP = smem + b * G::STAGE_FL;
@@ -326,11 +348,6 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
             }
         }
         __syncthreads();
-        // every thread is done with shot k-1: refill its buffer with shot k+1
-        // (its generic-proxy writes were fenced at the end of shot k-1)
-        if (threadIdx.x == 0 && k >= 1 && k + 1 < ns)
-            stage_loads<R>(mP, mVX, mVZ, smem + (b ^ 1) * G::STAGE_FL, &bars[b ^ 1], G::STAGE_BYTES, x0, z0,
-                           s + 1, G::P_FL, G::VX_FL);
 
         if (FS && !fast) {
             // p[fs-1] = -p[fs+1] inside the rectangle
@@ -461,10 +478,8 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                 if ((en.w & 2) && A.tr_vz) A.tr_vz[t] = sVZ[(en.x + 2 * R) * RW + cc];
             }
         }
-        // order this iteration's generic-proxy shared-memory writes before the
-        // TMA that refills the buffer (issued after the next iteration's
-        // mid-shot barrier)
-        fence_proxy_async_smem();
+        if (k + 2 < ns && last_warp_of_shot(&s_done, lane))
+            stage_loads<R>(mP, mVX, mVZ, sP, &bars[b], G::STAGE_BYTES, x0, z0, s + 2, G::P_FL, G::VX_FL);
     }
 
     if (ENERGY && vlane && A.energy) {
