@@ -316,6 +316,21 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                 }
             }
         }
+        // the slow path's damping of this warp's rows: on its way during the
+        // barrier where the registers allow it (as in the forward)
+        constexpr bool PRE = !CPML && !RHO && R == 2;
+        float4 d1[G::LV], d2[G::LV], d3[G::LV];
+        if (PRE && !fast) {
+#pragma unroll
+            for (int u = 0; u < G::LV; ++u) {
+                const int gz = z0 + vb + u;
+                const bool on = vlane && u < vcnt && gz < g.Nz && gx0 < g.Nx;
+                const long long o = (long long)gz * g.pitch + gx0;
+                d1[u] = ldg4_if(on, A.k1 + o);
+                d2[u] = ldg4_if(on, A.k2 + o);
+                d3[u] = ldg4_if(on, A.k3 + o);
+            }
+        }
         __syncthreads();
         if (A.grad_wavelet && threadIdx.x == 0) {
             // the tile that owns the source cell: mu_p / a1 there is lambda_p
@@ -414,8 +429,8 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                             }
                             if (any_v) {
                                 // no damping with CPML
-                                const float4 k2 = CPML ? zero4() : ldg4(A.k2 + o);
-                                const float4 k3 = CPML ? zero4() : ldg4(A.k3 + o);
+                                const float4 k2 = CPML ? zero4() : PRE ? d2[u] : ldg4(A.k2 + o);
+                                const float4 k3 = CPML ? zero4() : PRE ? d3[u] : ldg4(A.k3 + o);
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
                                     const int gx = gx0 + q;
@@ -436,7 +451,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                                 }
                             }
                             if (any_p) {
-                                const float4 k1 = CPML ? zero4() : ldg4(A.k1 + o);
+                                const float4 k1 = CPML ? zero4() : PRE ? d1[u] : ldg4(A.k1 + o);
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
                                     const int gx = gx0 + q;

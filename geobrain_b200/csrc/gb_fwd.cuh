@@ -247,6 +247,30 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
     for (int k = 0; k < ns; ++k) {
         const int s = s0 + k;
         const int b = k & 1;
+        // what the slow path reads beside the stage for this warp's p rows
+        // (damping, or the memory variables of a layer): on its way during the
+        // wait where the registers allow it.  (32 shots of 464 x 1320, a third
+        // of the tiles slow: R = 2 103.4 -> 98.0 us a step; at R = 4 the taps
+        // fill the registers and it went 115.4 -> 118.4.)
+        constexpr bool PRE = R == 2;
+        float4 d1[G::LP], e1[CPML ? G::LP : 1];
+        const auto load_p = [&](int u, bool on, long long o) {
+            if constexpr (CPML) {
+                const float *ps = A.psi_in + (long long)s * 4 * g.plane + o;
+                d1[u] = ldg4_if(on && any4(lds4(cp.ax[0] + 4 * lane + 4)), ps);
+                e1[u] = ldg4_if(on && cp.az[0][rb + u + R] != 0.f, ps + g.plane);
+            } else {
+                d1[u] = ldg4_if(on, A.k1 + o);
+            }
+        };
+        if (PRE && !fast) {
+#pragma unroll
+            for (int u = 0; u < G::LP; ++u) {
+                const int gz = z0 - R + rb + u;
+                load_p(u, u < rc && gz >= g.p_r0 && gz <= g.p_r1 && gx0 + 3 >= g.p_c0 && gx0 <= g.p_c1,
+                       (long long)gz * g.pitch + gx0);
+            }
+        }
         // every thread waits (bounded) for this shot's stage; no CTA barrier
         // here: shot k-1's buffer is refilled by the last warp to finish that
         // shot.  A give-up sets the status word and the launch runs on
@@ -293,13 +317,14 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                         if (row_in && (gx0 + 3 >= g.p_c0) && (gx0 <= g.p_c1)) {
                             const long long o = (long long)gz * g.pitch + gx0;
                             float4 img;
+                            if (!PRE) load_p(u, true, o);
                             if constexpr (CPML) {
                                 // psi' = b psi + a d, p' = p - a1 ((Dx + psi_x') + (Dz + psi_z'))
                                 const float bz = cp.bz[0][r + R], az = cp.az[0][r + R];
                                 const float4 bx = lds4(cp.bx[0] + 4 * lane + 4), ax = lds4(cp.ax[0] + 4 * lane + 4);
                                 const bool lx = any4(ax), lz = az != 0.f;
                                 const long long po = (long long)s * 4 * g.plane + o;
-                                const float4 ox = ldg4_if(lx, A.psi_in + po), oz = ldg4_if(lz, A.psi_in + po + g.plane);
+                                const float4 ox = d1[u], oz = e1[u];
                                 float Dx[4], Dz[4];
                                 divergence4_split<R>(sVX + r * VXW, lane, wz, u, g.c, Dx, Dz);
                                 float4 nx = ox, nz = oz;
@@ -320,13 +345,12 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                                 if (lz) stg4(A.psi_out + po + g.plane, nz);
                             } else {
                                 divergence4<R>(sVX + r * VXW, lane, wz, u, g.c, D);
-                                const float4 k1 = ldg4(A.k1 + o);
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
                                     const int gx = gx0 + q;
                                     const bool m = gx >= g.p_c0 && gx <= g.p_c1;
                                     at(img, q) = m ? -D[q] : 0.f;
-                                    if (m) at(pv, q) = __fmaf_rn(-at(a1, q), D[q], (1.f - at(k1, q)) * at(pv, q));
+                                    if (m) at(pv, q) = __fmaf_rn(-at(a1, q), D[q], (1.f - at(d1[u], q)) * at(pv, q));
                                 }
                             }
                             if (tile_cell && imaging)
@@ -345,6 +369,25 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                     }
                     sts4(sP + r * RW + 4 * lane, pv);
                 }
+            }
+        }
+        // and for its v rows, during the barrier
+        float4 d2[G::LV], d3[G::LV];
+        const auto load_v = [&](int u, bool on, long long o) {
+            if constexpr (CPML) {
+                const float *ps = A.psi_in + (long long)s * 4 * g.plane + o;
+                d2[u] = ldg4_if(on && any4(lds4(cp.ax[1] + 4 * lane + 4)), ps + 2 * g.plane);
+                d3[u] = ldg4_if(on && cp.az[1][vb + u + 2 * R] != 0.f, ps + 3 * g.plane);
+            } else {
+                d2[u] = ldg4_if(on, A.k2 + o);
+                d3[u] = ldg4_if(on, A.k3 + o);
+            }
+        };
+        if (PRE && !fast) {
+#pragma unroll
+            for (int u = 0; u < G::LV; ++u) {
+                const int gz = z0 + vb + u;
+                load_v(u, vlane && u < vcnt && gz < g.Nz && gx0 < g.Nx, (long long)gz * g.pitch + gx0);
             }
         }
         __syncthreads();
@@ -394,14 +437,14 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                             const bool vz_row = gz >= g.vz_r0 && gz <= g.vz_r1;
                             const bool need = (vx_row && gx0 + 3 >= g.vx_c0 && gx0 <= g.vx_c1) ||
                                               (vz_row && gx0 + 3 >= g.vz_c0 && gx0 <= g.vz_c1);
+                            if (!PRE) load_v(u, need, o);
                             if constexpr (CPML) {
                                 // psi' = b psi + a G, v' = v - a2 (G + psi')
                                 const float bz = cp.bz[1][rv + 2 * R], az = cp.az[1][rv + 2 * R];
                                 const float4 bx = lds4(cp.bx[1] + 4 * lane + 4), ax = lds4(cp.ax[1] + 4 * lane + 4);
                                 const bool lx = need && any4(ax), lz = need && az != 0.f;
                                 const long long po = (long long)s * 4 * g.plane + o;
-                                const float4 ox = ldg4_if(lx, A.psi_in + po + 2 * g.plane),
-                                             oz = ldg4_if(lz, A.psi_in + po + 3 * g.plane);
+                                const float4 ox = d2[u], oz = d3[u];
                                 float4 nx = ox, nz = oz;
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
@@ -420,17 +463,15 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                                 if (lx) stg4(A.psi_out + po + 2 * g.plane, nx);
                                 if (lz) stg4(A.psi_out + po + 3 * g.plane, nz);
                             } else if (need) {
-                                const float4 k2 = ldg4(A.k2 + o);
-                                const float4 k3 = ldg4(A.k3 + o);
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
                                     const int gx = gx0 + q;
                                     if (vx_row && gx >= g.vx_c0 && gx <= g.vx_c1) {
-                                        at(vx, q) = __fmaf_rn(-at(a2, q), Dx[q], (1.f - at(k2, q)) * at(vx, q));
+                                        at(vx, q) = __fmaf_rn(-at(a2, q), Dx[q], (1.f - at(d2[u], q)) * at(vx, q));
                                         at(jx, q) = Dx[q];
                                     }
                                     if (vz_row && gx >= g.vz_c0 && gx <= g.vz_c1) {
-                                        at(vz, q) = __fmaf_rn(-at(a2, q), Dz[q], (1.f - at(k3, q)) * at(vz, q));
+                                        at(vz, q) = __fmaf_rn(-at(a2, q), Dz[q], (1.f - at(d3[u], q)) * at(vz, q));
                                         at(jz, q) = Dz[q];
                                     }
                                 }
