@@ -396,19 +396,31 @@ struct gb_plan {
         return n;
     }
 
-    // Enough CTAs to fill the GPU several times over, as few groups as that
-    // allows (each group re-reads the coefficient tiles and adds its own
-    // energy / gradient partial sums); at most 8 shots per CTA.
+    // Shots per CTA: the S shots go to g groups of about equal size, at most 8
+    // shots each.  A CTA costs its shots and about 0.82 of a shot (its
+    // coefficient tiles, and the energy or gradient partial sums that each
+    // group adds at each step), so fewer groups are less work; and a step of
+    // tiles x g CTAs fills the 296 resident slots only when there are more of
+    // them, as the groups' streams cover each other's ends: measured, 0.5 of
+    // the rate at 160 CTAs, 0.75 at 300, 0.89 at 450, 1 from 592 on.
+    // Gradient, ms, against the fewest groups that give 592 CTAs (all filled
+    // up but the last): 128 x 240, 40 shots, 300 steps 7.87 -> 7.33 (2 shots
+    // per CTA for 1); 240 x 540, 12 shots, 200 steps 6.68 -> 5.60 (2 for 1);
+    // 460 x 1260, 8 shots, 150 steps, CPML 25.3 -> 17.7 (4 + 4 for 7 + 1).
     int default_spc() const
     {
         const int S = d.n_shots;
-        int best = S;
-        for (int spc_try = S; spc_try >= 1; --spc_try) {
-            const long long ctas = (long long)n_tiles * ((S + spc_try - 1) / spc_try);
-            best = spc_try;
-            if (ctas >= 4 * 148) break;
+        int best = 0;
+        double best_cost = 0.0;
+        for (int groups = (S + 7) / 8; groups <= S; ++groups) {
+            const int per = (S + groups - 1) / groups;
+            if ((S + per - 1) / per != groups) continue;
+            const double ctas = (double)n_tiles * groups;
+            const double fill = ctas >= 592.0 ? 1.0 : ctas >= 296.0 ? std::pow(ctas / 592.0, 0.4) : 0.758 * ctas / 296.0;
+            const double cost = (0.82 * groups + S) / fill;
+            if (!best || cost < best_cost) best = per, best_cost = cost;
         }
-        return std::max(1, std::min(best, 8));
+        return std::max(1, best);
     }
 
     StepGeom geom() const
