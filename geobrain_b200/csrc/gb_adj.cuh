@@ -183,8 +183,8 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
     }
 
     const int gx0 = x0 - 4 + 4 * lane;
-    const int rb = warp * G::LP, rc = min(G::LP, G::PR - rb);
-    const int vb = warp * G::LV, vcnt = min(G::LV, TZ - vb);
+    const int rb = warp * G::LP, rc = G::PR == NWARP * G::LP ? G::LP : min(G::LP, G::PR - rb);
+    const int vb = warp * G::LV, vcnt = TZ == NWARP * G::LV ? G::LV : min(G::LV, TZ - vb);
     const bool vlane = lane >= 1 && lane <= 30;
 
     // per-thread partial sums over this CTA's shots (tile cells)

@@ -234,8 +234,8 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
     }
 
     const int gx0 = x0 - 4 + 4 * lane;   // first of this thread's 4 columns
-    const int rb = warp * G::LP, rc = min(G::LP, G::PR - rb);      // p-stage rows of this warp
-    const int vb = warp * G::LV, vcnt = min(G::LV, TZ - vb);       // v-stage rows of this warp
+    const int rb = warp * G::LP, rc = G::PR == NWARP * G::LP ? G::LP : min(G::LP, G::PR - rb);      // p-stage rows of this warp
+    const int vb = warp * G::LV, vcnt = TZ == NWARP * G::LV ? G::LV : min(G::LV, TZ - vb);       // v-stage rows of this warp
     const bool vlane = lane >= 1 && lane <= 30;
 
     float4 e_p[G::LV], e_vx[G::LV], e_vz[G::LV];
