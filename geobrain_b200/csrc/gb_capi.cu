@@ -336,12 +336,34 @@ struct gb_plan {
     // tiles fit on the SMs at once (few shots or a small grid: the cases
     // where the per-step tile kernel is launch- and latency-bound), with the
     // two exchanges through global memory and the smallest tile height that
-    // fits (the most CTAs).  The cluster exchange (16 CTAs a shot at most)
+    // fits (the most CTAs).  At 8th order 4-row tiles are all boundary twice
+    // over (each row goes up and down: 140 x 240, 1000 steps 3.74 ms against
+    // 3.05 with 8 rows) and 12-row tiles with 8 warps are slower than 16 with
+    // 16 (3.77, 3.54): both are left out.  The cluster exchange (16 CTAs a shot at most)
     // and one exchange a step (which sends twice the cells to eight
     // neighbours and updates p on twice the rows) measured no faster on the
     // 100 x 200 grid; they run when asked for.  More shots keep the tile
     // kernel.
     bool res_single_ok() const { return R == 2 && !d.free_surface; }
+    // A gradient runs the resident kernels when it keeps every step's imaging
+    // fields (no checkpoints to write or restart from) and edge cells go
+    // through global memory; its adjoint when also the residuals are of the
+    // pressure alone and each shot has a group (partial sums) of its own,
+    // which few shots on few tiles always have.  Without step graphs a
+    // gradient is one plain launch per step and group, which a caller's own
+    // stream capture can take; it stays so.  One shot of 140 x 240, 600
+    // steps, 4th order: 6.75 ms with the tile kernels, 5.02 with the resident
+    // forward, 3.40 with both; 16 shots of it (36-row tiles on
+    // all SMs) 6.37 and 4.18 for 400 steps; one shot of 460 x 1260, 200 steps,
+    // 8th order, 4.63 and 2.77.
+    bool res_gradient(int cached_steps) const
+    {
+        return res_tz > 0 && res_exchange() == 0 && graph_steps > 0 && !cpml && cached_steps == d.nt;
+    }
+    bool res_adjoint(int cached_steps, const float *res_p, const float *res_vx, const float *res_vz) const
+    {
+        return res_gradient(cached_steps) && res_p && !res_vx && !res_vz && n_groups == d.n_shots;
+    }
     void res_choose()
     {
         res_tz = 0;
@@ -361,6 +383,7 @@ struct gb_plan {
                 const long long n = (long long)((Nx + TX - 1) / TX) * ((Nz + tz - 1) / tz);
                 if (cl && n > kMaxClusterTiles) continue;
                 if (res_mode < 0 && n * d.n_shots > sms) continue;
+                if (res_mode < 0 && !res_tz_req && R == 4 && (tz == 4 || tz == 12)) continue;
                 best = tz;
                 res_cluster = cl;
                 res_single = sx;
@@ -487,7 +510,7 @@ Layout layout(const gb_plan *p, int with_gradient = 0, int checkpoint_every = 0,
         L.cpml = o; o = align256(o + (4 * (size_t)p->Nz + 4 * (size_t)p->pitch) * 4);
         L.psi = o; o = align256(o + 2 * S * 4 * p->plane * 4);   // two levels of the memory variables
     }
-    if (p->res_tz > 0 && with_gradient == 0) {
+    if (p->res_tz > 0) {
         const ResidentKernel k = resident_kernel(p->R, p->res_tz, p->res_single ? 2 : 0);
         L.res_ptr = o; o = align256(o + (p->res_n + 1) * 4);
         L.res_ent = o; o = align256(o + std::max<size_t>(p->d.n_rcv, 1) * 16);
@@ -1060,20 +1083,14 @@ int check_store(const gb_plan *P, const gb_grad_store *store)
     return GB_OK;
 }
 
-// Plain forward by the resident kernel: cooperative launches of res_n tiles x
-// res_shots shots, each running a chunk of steps with the state in shared
-// memory (chunks end where a snapshot of shot 0 is due).  The state starts
-// and ends in buf (level 0 of the workspace's fields).
-int forward_resident(gb_plan *P, const Layout &L, char *ws, const Setup &Su, float *buf, float *energy,
-                     bool want_energy, const float *wavelet, float *trace_p, float *trace_vx, float *trace_vz,
-                     int32_t snapshot_every, float *snapshots, cudaStream_t st)
+// What a resident kernel's launches share: its receivers, exchange strips
+// and, with a store, the imaging fields of every step.
+int resident_args(gb_plan *P, const Layout &L, char *ws, const Setup &Su, const ResidentKernel &K,
+                  const gb_grad_store *store, cudaStream_t st, ResArgs *out)
 {
     const gb_model_desc &d = P->d;
     const int S = d.n_shots;
-    const ResidentKernel K = resident_kernel(P->R, P->res_tz, P->res_exchange());
-    if (!K.fn) return fail(GB_E_UNSUPPORTED, "no resident kernel for this tile height");
     GB_CUDA(cudaFuncSetAttribute(K.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K.smem));
-    if (P->res_cluster && P->res_n > 8) GB_CUDA(cudaFuncSetAttribute(K.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     int *d_ptr = reinterpret_cast<int *>(ws + L.res_ptr);
     int4 *d_ent = reinterpret_cast<int4 *>(ws + L.res_ent);
     GB_CUDA(cudaMemcpyAsync(d_ptr, P->res_ptr.data(), (P->res_n + 1) * 4, cudaMemcpyHostToDevice, st));
@@ -1086,17 +1103,69 @@ int forward_resident(gb_plan *P, const Layout &L, char *ws, const Setup &Su, flo
     A.tiles_x = P->res_tiles_x;
     A.tiles_z = P->res_tiles_z;
     A.n_tiles = P->res_n;
-    A.energy = want_energy ? 1 : 0;
     A.free_surface = d.free_surface ? 1 : 0;
     A.a1 = Su.a1; A.k1 = Su.k1; A.a2 = Su.a2; A.k2 = Su.k2; A.k3 = Su.k3;
-    A.state = buf;
     A.src_z = Su.d_src; A.src_x = Su.d_src + S;
-    A.wavelet = wavelet;
     A.rcv_ptr = d_ptr; A.rcv_ent = d_ent;
-    A.tr_p = trace_p; A.tr_vx = trace_vx; A.tr_vz = trace_vz;
-    A.energy_map = want_energy ? energy : nullptr;
     A.xbuf = reinterpret_cast<uint2 *>(ws + L.res_x);
     A.err = Su.err;
+    if (store) {
+        A.img = reinterpret_cast<char *>(store->imaging);
+        A.img_fmt = store->imaging_format;
+        A.img_field_stride = (long long)S * P->plane;
+        A.img_step = A.img_field_stride * (store->with_rho ? 3 : 1);
+    }
+    *out = A;
+    return GB_OK;
+}
+
+// The adjoint of every step by the resident kernel: the gradients' sums of
+// shot s go to plane s of G1, C1 (and G2, C2).
+int adjoint_resident(gb_plan *P, const Layout &L, char *ws, const Setup &Su, const gb_grad_store *store,
+                     const float *res_p, float *G1, float *C1, float *G2, float *C2, float *grad_wavelet,
+                     cudaStream_t st)
+{
+    const ResidentKernel K = resident_adj_kernel_for(P->R, P->res_tz, G2 != nullptr);
+    if (!K.fn) return fail(GB_E_UNSUPPORTED, "no resident kernel for this tile height");
+    ResArgs A;
+    if (int rc = resident_args(P, L, ws, Su, K, store, st, &A)) return rc;
+    A.res_p = res_p;
+    A.G1 = G1; A.C1 = C1; A.G2 = G2; A.C2 = C2;
+    A.grad_wavelet = grad_wavelet;
+    A.it0 = 0;
+    A.it1 = P->d.nt;
+    for (int s0 = 0; s0 < P->d.n_shots; s0 += P->res_shots) {
+        A.shot0 = s0;
+        void *args[] = {(void *)&A};
+        GB_CUDA(cudaLaunchCooperativeKernel(K.fn, dim3((unsigned)(P->res_n * std::min(P->res_shots, P->d.n_shots - s0))),
+                                            dim3(K.threads), args, K.smem, st));
+        ++P->launches;
+        ++P->api_launches;
+    }
+    return GB_OK;
+}
+
+// Plain forward by the resident kernel: cooperative launches of res_n tiles x
+// res_shots shots, each running a chunk of steps with the state in shared
+// memory (chunks end where a snapshot of shot 0 is due).  The state starts
+// and ends in buf (level 0 of the workspace's fields).
+int forward_resident(gb_plan *P, const Layout &L, char *ws, const Setup &Su, float *buf, float *energy,
+                     bool want_energy, const float *wavelet, float *trace_p, float *trace_vx, float *trace_vz,
+                     int32_t snapshot_every, float *snapshots, const gb_grad_store *store, cudaStream_t st)
+{
+    const gb_model_desc &d = P->d;
+    const int S = d.n_shots;
+    const ResidentKernel K = store ? resident_img_kernel(P->R, P->res_tz, store->with_rho ? 2 : 1)
+                                   : resident_kernel(P->R, P->res_tz, P->res_exchange());
+    if (!K.fn) return fail(GB_E_UNSUPPORTED, "no resident kernel for this tile height");
+    if (P->res_cluster && P->res_n > 8) GB_CUDA(cudaFuncSetAttribute(K.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    ResArgs A;
+    if (int rc = resident_args(P, L, ws, Su, K, store, st, &A)) return rc;
+    A.energy = want_energy ? 1 : 0;
+    A.state = buf;
+    A.wavelet = wavelet;
+    A.tr_p = trace_p; A.tr_vx = trace_vx; A.tr_vz = trace_vz;
+    A.energy_map = want_energy ? energy : nullptr;
     int snap_i = 0;
     for (int s0 = 0; s0 < S; s0 += P->res_shots) {
         const int ns = std::min(P->res_shots, S - s0);
@@ -1430,10 +1499,10 @@ int gb_forward(gb_plan *P, const float *vp, const float *rho, const float *damp,
     GB_CUDA(cudaMemsetAsync(buf[1], 0, (size_t)S * 3 * P->plane * 4, st));
     if (want_energy) GB_CUDA(cudaMemsetAsync(energy, 0, 3 * P->plane * 4, st));
 
-    if (P->res_tz > 0 && !store && !P->cpml) {
+    if (store ? P->res_gradient(store->cached_steps) : P->res_tz > 0 && !P->cpml) {
         P->phase_steps[0] += d.nt;
         if (int rc = forward_resident(P, L, ws, Su, buf[0], energy, want_energy, wavelet, trace_p, trace_vx,
-                                      trace_vz, snapshot_every, snapshots, st))
+                                      trace_vz, snapshot_every, snapshots, store, st))
             return rc;
         float *eo[3] = {energy_p, energy_vx, energy_vz};
         for (int f = 0; f < 3; ++f)
@@ -1828,12 +1897,25 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
     GB_CUDA(cudaMemcpyAsync(d_aptr, P->arcv_ptr.data(), (P->n_tiles + 1) * 4, cudaMemcpyHostToDevice, st));
     if (!P->arcv_ent.empty())
         GB_CUDA(cudaMemcpyAsync(d_aent, P->arcv_ent.data(), P->arcv_ent.size() * 16, cudaMemcpyHostToDevice, st));
-    GB_CUDA(cudaMemsetAsync(mu[0], 0, 2 * state_fl * 4, st));
+    const bool resident = P->res_adjoint(store->cached_steps, res_p, res_vx, res_vz);
+    if (!resident) GB_CUDA(cudaMemsetAsync(mu[0], 0, 2 * state_fl * 4, st));
     GB_CUDA(cudaMemsetAsync(G1, 0, (size_t)P->n_groups * P->plane * 4, st));
     GB_CUDA(cudaMemsetAsync(C1, 0, (size_t)P->n_groups * P->plane * 4, st));
     if (G2) {
         GB_CUDA(cudaMemsetAsync(G2, 0, (size_t)P->n_groups * P->plane * 4, st));
         GB_CUDA(cudaMemsetAsync(C2, 0, (size_t)P->n_groups * P->plane * 4, st));
+    }
+
+    if (resident) {
+        P->mark(2, true, st);
+        P->phase_steps[2] += d.nt;
+        if (int rc = adjoint_resident(P, L, ws, Su, store, res_p, G1, C1, G2, C2, grad_wavelet, st)) return rc;
+        P->mark(2, false, st);
+        grad_finish_kernel<<<4 * 148, 256, 0, st>>>(vp, rho, G1, C1, G2, C2, P->n_groups, P->plane, d.nz, d.nx, d.nabc,
+                                                    P->pitch, grad_vp, grad_rho);
+        GB_CUDA(cudaGetLastError());
+        ++P->launches;
+        return GB_OK;
     }
 
     float *eta[2] = {nullptr, nullptr};

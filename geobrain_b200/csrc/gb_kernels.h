@@ -56,6 +56,11 @@ struct ResidentKernel {
 // the neighbours' edge rows and columns (gb_resident_sx.cuh: 4th order, no
 // free surface).
 ResidentKernel resident_kernel(int R, int tz, int exchange);
+// The forward through global memory (exchange 0) that also writes the imaging
+// fields, img 1 or 2.  gb_pick_resident_img.cu.
+ResidentKernel resident_img_kernel(int R, int tz, int img);
+// resident_adj_kernel<R, NW, TZ, RHO> (gb_resident_adj.cuh).  gb_pick_resident_adj.cu.
+ResidentKernel resident_adj_kernel_for(int R, int tz, bool rho);
 
 }  // namespace host
 }  // namespace gb

@@ -99,7 +99,25 @@ struct ResArgs {
     float *energy_map;                // [3][plane] padded accumulators (with energy)
     uint2 *xbuf;                      // [S][n_tiles][kResParts][PART] (value, tag) words, zero before a run
     int *err;
+    // imaging fields of every step (img_fmt, kImg*), img_step elements a step
+    // and img_field_stride between a step's fields: written by the forward
+    // with IMG > 0, read by the adjoint
+    char *img;
+    long long img_step, img_field_stride;
+    int img_fmt;
+    // adjoint only: dL/d(trace p) [S][nt][n_rcv], the gradients' sums and
+    // compensations [S][plane] (G2, C2 with RHO), dL/d(wavelet) or null
+    const float *res_p;
+    float *G1, *C1, *G2, *C2;
+    float *grad_wavelet;
 };
+
+// Step `it` of the imaging fields.
+__device__ __forceinline__ float *res_img_step(const ResArgs &A, int it)
+{
+    const int es = A.img_fmt == kImgBF16 ? 2 : A.img_fmt == kImgF24 ? 3 : 4;
+    return reinterpret_cast<float *>(A.img + (long long)it * A.img_step * es);
+}
 
 // Plain (coherent) 16-byte global load, for state another kernel wrote.
 __device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
@@ -200,9 +218,10 @@ struct ResCtx {
 // Pressure update of the 4 cells of rect row r, lane l (acoustic_2d.py
 // :211-237), as the tile kernel computes it; wz[u + R] is vz row r.
 // Returns the new values (also stored).
-template <int R>
+// IMG > 0: -div(v) goes to the step's imaging fields `img` where p is updated.
+template <int R, int IMG = 0>
 __device__ __forceinline__ float4 res_p_cells(const ResArgs &A, const ResCtx &C, int r, int l, const float4 *wz, int u,
-                                              int it)
+                                              int it, float *img = nullptr)
 {
     const StepGeom &g = A.g;
     float4 pv = lds4(C.sP + r * RS + 4 * l);
@@ -218,6 +237,12 @@ __device__ __forceinline__ float4 res_p_cells(const ResArgs &A, const ResCtx &C,
         for (int q = 0; q < 4; ++q) at(pv, q) = __fmaf_rn(-at(a1, q), D[q], at(d1, q) * at(pv, q));
     }
     const int gx0 = C.x0 - 4 + 4 * l;
+    if (IMG > 0 && C.z0 - R + r < g.Nz && gx0 < g.Nx) {
+        float4 v;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) at(v, q) = at(a1, q) != 0.f ? -D[q] : 0.f;
+        store_img4(img, (long long)C.s * g.plane + (long long)(C.z0 - R + r) * g.pitch + gx0, A.img_fmt, v);
+    }
     if (C.z0 - R + r == C.sz && C.sx >= gx0 && C.sx < gx0 + 4) {
         // p + dt * w, rounded after the product and after the sum (acoustic_2d.py:230-233)
         const float amp = __fmul_rn(g.dt, A.wavelet[(long long)C.s * g.nt + it]);
@@ -234,9 +259,10 @@ __device__ __forceinline__ float4 res_p_cells(const ResArgs &A, const ResCtx &C,
 // Velocity update of the 4 cells of rect row r, lane l (acoustic_2d.py
 // :244-265), as the tile kernel computes it; wp[u + R] is p row r + 1.
 // Returns the new vx and vz (also stored).
-template <int R>
+// IMG == 2: dx(p) and dz(p) go to the imaging fields where vx and vz are updated.
+template <int R, int IMG = 0>
 __device__ __forceinline__ void res_v_cells(const ResArgs &A, const ResCtx &C, int r, int l, const float4 *wp, int u,
-                                            float4 &vx, float4 &vz)
+                                            float4 &vx, float4 &vz, float *img = nullptr)
 {
     const StepGeom &g = A.g;
     float Dx[4], Dz[4];
@@ -263,6 +289,19 @@ __device__ __forceinline__ void res_v_cells(const ResArgs &A, const ResCtx &C, i
     }
     sts4(C.sVX + r * RS + 4 * l, vx);
     sts4(C.sVZ + r * RS + 4 * l, vz);
+    const int gx0 = C.x0 - 4 + 4 * l;
+    if (IMG == 2 && C.z0 - R + r < g.Nz && gx0 < g.Nx) {
+        const float4 az = lds4(C.cA2Z + o);
+        float4 jx, jz;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            at(jx, q) = at(ax, q) != 0.f ? Dx[q] : 0.f;
+            at(jz, q) = at(az, q) != 0.f ? Dz[q] : 0.f;
+        }
+        const long long io = (long long)C.s * g.plane + (long long)(C.z0 - R + r) * g.pitch + gx0;
+        store_img4(img, io + A.img_field_stride, A.img_fmt, jx);
+        store_img4(img, io + 2 * A.img_field_stride, A.img_fmt, jz);
+    }
 }
 
 // Boundary item i -> (rect row, lane): the boundary rows with lanes 1..30,
@@ -393,9 +432,60 @@ __device__ __forceinline__ bool res_receive(float *rows_f, float *cols_f, const 
     return __syncthreads_and(ok);
 }
 
+// The coefficients of the owned rows with the update masks and the damping
+// folded in, into the planes at cf.  Returns (to every thread, after a
+// barrier) whether the tile has no masks and no damping.
+template <int R, int NW, int TZ>
+__device__ __forceinline__ bool res_load_coef(const ResArgs &A, float *cf, int z0, int x0)
+{
+    using G = ResGeo<R, NW, TZ>;
+    const StepGeom &g = A.g;
+    bool damped = false;
+    for (int e = threadIdx.x; e < TZ * 32; e += G::NTH) {
+        const int r = e >> 5, l = e & 31;
+        const int gz = z0 + r, gx0 = x0 - 4 + 4 * l;
+        const bool in = gz < g.Nz && gx0 >= 0 && gx0 < g.pitch;
+        const long long o = (long long)gz * g.pitch + gx0;
+        const float4 a1 = in ? ldg4(A.a1 + o) : zero4(), a2 = in ? ldg4(A.a2 + o) : zero4();
+        const float4 k1 = in ? ldg4(A.k1 + o) : zero4(), k2 = in ? ldg4(A.k2 + o) : zero4();
+        const float4 k3 = in ? ldg4(A.k3 + o) : zero4();
+        float4 a1m, d1, a2x, d2, a2z, d3;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int gx = gx0 + q;
+            const bool pm = gz >= g.p_r0 && gz <= g.p_r1 && gx >= g.p_c0 && gx <= g.p_c1;
+            const bool xm = gz >= g.vx_r0 && gz <= g.vx_r1 && gx >= g.vx_c0 && gx <= g.vx_c1;
+            const bool zm = gz >= g.vz_r0 && gz <= g.vz_r1 && gx >= g.vz_c0 && gx <= g.vz_c1;
+            at(a1m, q) = pm ? at(a1, q) : 0.f;
+            at(d1, q) = pm ? 1.f - at(k1, q) : 1.f;
+            at(a2x, q) = xm ? at(a2, q) : 0.f;
+            at(d2, q) = xm ? 1.f - at(k2, q) : 1.f;
+            at(a2z, q) = zm ? at(a2, q) : 0.f;
+            at(d3, q) = zm ? 1.f - at(k3, q) : 1.f;
+        }
+        const int c = r * RS + 4 * l;
+        sts4(cf + c, a1m);
+        sts4(cf + G::CF + c, d1);
+        sts4(cf + 2 * G::CF + c, a2x);
+        sts4(cf + 3 * G::CF + c, d2);
+        sts4(cf + 4 * G::CF + c, a2z);
+        sts4(cf + 5 * G::CF + c, d3);
+        if (l >= 1 && l <= 30)
+            damped |= k1.x != 0.f || k1.y != 0.f || k1.z != 0.f || k1.w != 0.f || k2.x != 0.f || k2.y != 0.f ||
+                      k2.z != 0.f || k2.w != 0.f || k3.x != 0.f || k3.y != 0.f || k3.z != 0.f || k3.w != 0.f;
+    }
+    // no masks anywhere on the owned cells, and no damping: the undamped update
+    const bool inside = z0 >= g.p_r0 && z0 + TZ - 1 <= g.p_r1 && x0 >= g.p_c0 && x0 + TX - 1 <= g.p_c1 &&
+                        z0 >= g.vx_r0 && z0 + TZ - 1 <= g.vx_r1 && x0 >= g.vx_c0 && x0 + TX - 1 <= g.vx_c1 &&
+                        z0 >= g.vz_r0 && z0 + TZ - 1 <= g.vz_r1 && x0 >= g.vz_c0 && x0 + TX - 1 <= g.vz_c1;
+    return !__syncthreads_or(damped) && inside;
+}
+
 // CL: exchange through distributed shared memory within one cluster per
 // shot (the launch's cluster is the shot's n_tiles CTAs, rank = tile).
-template <int R, int NW, int TZ, bool CL>
+// IMG: 0 no imaging fields; 1 store I = -div(v^n); 2 also Jx, Jz (as in the
+// tile kernel, to the bit).
+template <int R, int NW, int TZ, bool CL, int IMG = 0>
 __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs A)
 {
     using G = ResGeo<R, NW, TZ>;
@@ -452,47 +542,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
         sts4(sVX + r * RS + 4 * l, in ? ld4(st + g.plane + o) : zero4());
         sts4(sVZ + r * RS + 4 * l, in ? ld4(st + 2 * g.plane + o) : zero4());
     }
-    // the coefficients of the owned rows with the update masks and the
-    // damping folded in
-    bool damped = false;
-    for (int e = threadIdx.x; e < TZ * 32; e += G::NTH) {
-        const int r = e >> 5, l = e & 31;
-        const int gz = z0 + r, gx0 = x0 - 4 + 4 * l;
-        const bool in = gz < g.Nz && gx0 >= 0 && gx0 < g.pitch;
-        const long long o = (long long)gz * g.pitch + gx0;
-        const float4 a1 = in ? ldg4(A.a1 + o) : zero4(), a2 = in ? ldg4(A.a2 + o) : zero4();
-        const float4 k1 = in ? ldg4(A.k1 + o) : zero4(), k2 = in ? ldg4(A.k2 + o) : zero4();
-        const float4 k3 = in ? ldg4(A.k3 + o) : zero4();
-        float4 a1m, d1, a2x, d2, a2z, d3;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int gx = gx0 + q;
-            const bool pm = gz >= g.p_r0 && gz <= g.p_r1 && gx >= g.p_c0 && gx <= g.p_c1;
-            const bool xm = gz >= g.vx_r0 && gz <= g.vx_r1 && gx >= g.vx_c0 && gx <= g.vx_c1;
-            const bool zm = gz >= g.vz_r0 && gz <= g.vz_r1 && gx >= g.vz_c0 && gx <= g.vz_c1;
-            at(a1m, q) = pm ? at(a1, q) : 0.f;
-            at(d1, q) = pm ? 1.f - at(k1, q) : 1.f;
-            at(a2x, q) = xm ? at(a2, q) : 0.f;
-            at(d2, q) = xm ? 1.f - at(k2, q) : 1.f;
-            at(a2z, q) = zm ? at(a2, q) : 0.f;
-            at(d3, q) = zm ? 1.f - at(k3, q) : 1.f;
-        }
-        const int c = r * RS + 4 * l;
-        sts4(cf + c, a1m);
-        sts4(cf + G::CF + c, d1);
-        sts4(cf + 2 * G::CF + c, a2x);
-        sts4(cf + 3 * G::CF + c, d2);
-        sts4(cf + 4 * G::CF + c, a2z);
-        sts4(cf + 5 * G::CF + c, d3);
-        if (l >= 1 && l <= 30)
-            damped |= k1.x != 0.f || k1.y != 0.f || k1.z != 0.f || k1.w != 0.f || k2.x != 0.f || k2.y != 0.f ||
-                      k2.z != 0.f || k2.w != 0.f || k3.x != 0.f || k3.y != 0.f || k3.z != 0.f || k3.w != 0.f;
-    }
-    // no masks anywhere on the owned cells, and no damping: the undamped update
-    const bool inside = z0 >= g.p_r0 && z0 + TZ - 1 <= g.p_r1 && x0 >= g.p_c0 && x0 + TX - 1 <= g.p_c1 &&
-                        z0 >= g.vx_r0 && z0 + TZ - 1 <= g.vx_r1 && x0 >= g.vx_c0 && x0 + TX - 1 <= g.vx_c1 &&
-                        z0 >= g.vz_r0 && z0 + TZ - 1 <= g.vz_r1 && x0 >= g.vz_c0 && x0 + TX - 1 <= g.vz_c1;
-    C.fast = !__syncthreads_or(damped) && inside;
+    C.fast = res_load_coef<R, NW, TZ>(A, cf, z0, x0);
     const int fs = g.fs;
     // free surface: rect row of the mirror row (the tiling keeps rows fs-1 .. fs+1 in one tile)
     const int rm = fs - 1 - (z0 - R);
@@ -527,6 +577,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
     if (CL) cluster_arrive();   // the first step's v exchange waits on this phase
 
     for (int it = A.it0; it < A.it1; ++it) {
+        float *const img = IMG > 0 ? res_img_step(A, it) : nullptr;
         // ---- p interior (reads the tile's own v only) ---------------------
         if (interior) {
             float4 wz[G::LI + 2 * R - 1];
@@ -534,7 +585,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
             for (int t = 0; t < G::LI + 2 * R - 1; ++t) wz[t] = lds4(sVZ + (ri - R + t) * RS + 4 * lane);
 #pragma unroll
             for (int u = 0; u < G::LI; ++u)
-                if (ri + u < TZ) res_p_cells<R>(A, C, ri + u, lane, wz, u, it);
+                if (ri + u < TZ) res_p_cells<R, IMG>(A, C, ri + u, lane, wz, u, it, img);
         }
         // ---- the neighbours' v boundary cells of the previous step ---------
         // (a mirror row arrives mirrored: its owner sends it after the mirror)
@@ -547,7 +598,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
             float4 wz[2 * R];
 #pragma unroll
             for (int t = 0; t < 2 * R; ++t) wz[t] = lds4(sVZ + (r - R + t) * RS + 4 * l);
-            const float4 pv = res_p_cells<R>(A, C, r, l, wz, 0, it);
+            const float4 pv = res_p_cells<R, IMG>(A, C, r, l, wz, 0, it, img);
             if (!(fs_own && r == rm)) res_send4<R, TZ, CL>(K, K.rP, 0, 2, true, true, r, l, pv, tag_p(it));
         }
         __syncthreads();
@@ -571,7 +622,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
             for (int u = 0; u < G::LI; ++u)
                 if (ri + u < TZ) {
                     float4 vx, vz;
-                    res_v_cells<R>(A, C, ri + u, lane, wp, u, vx, vz);
+                    res_v_cells<R, IMG>(A, C, ri + u, lane, wp, u, vx, vz, img);
                 }
         }
         // ---- the neighbours' p boundary cells ------------------------------
@@ -586,7 +637,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
 #pragma unroll
             for (int t = 0; t < 2 * R; ++t) wp[t] = lds4(sP + (r - R + 1 + t) * RS + 4 * l);
             float4 vx, vz;
-            res_v_cells<R>(A, C, r, l, wp, 0, vx, vz);
+            res_v_cells<R, IMG>(A, C, r, l, wp, 0, vx, vz, img);
             if (send_v) {
                 res_send4<R, TZ, CL>(K, K.rVZ, 4, 6, !(fs_own && r == rm), false, r, l, vz, tag_v(it));
                 res_send4<R, TZ, CL>(K, K.rVX, 4, 6, false, true, r, l, vx, tag_v(it));
