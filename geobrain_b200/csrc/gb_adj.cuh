@@ -195,6 +195,9 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
         acc2[u] = zero4();
     }
 
+    // (a batch's arguments are in shared memory, where each barrier would have
+    // them read again)
+    const float tap[4] = {g.c[0], g.c[1], g.c[2], g.c[3]};
     for (int k = 0; k < ns; ++k) {
         const int s = s0 + k;
         const int b = k & 1;
@@ -273,7 +276,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                     const float4 a1 = lds4(sA1 + r * RW + 4 * lane);
                     float D[4];
                     if (fast) {
-                        divergence4<R>(sVX + r * VXW, lane, wz, u, g.c, D);
+                        divergence4<R>(sVX + r * VXW, lane, wz, u, tap, D);
 #pragma unroll
                         for (int q = 0; q < 4; ++q) at(pv, q) = __fmaf_rn(at(a1, q), D[q], at(pv, q));
                     } else {
@@ -291,9 +294,9 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                                 for (int t = 0; t < 3; ++t)
                                     e[t] = cpml_mix(lds4(sVX + r * VXW + 4 * lane + 4 * t), lds4(cp.bx[1] + 4 * lane + 4 * t),
                                                     lds4(cp.ax[1] + 4 * lane + 4 * t), h[t]);
-                                divergence4_of<R>(e[0], e[1], e[2], wz, u, g.c, D);
+                                divergence4_of<R>(e[0], e[1], e[2], wz, u, tap, D);
                             } else {
-                                divergence4<R>(sVX + r * VXW, lane, wz, u, g.c, D);
+                                divergence4<R>(sVX + r * VXW, lane, wz, u, tap, D);
                             }
 #pragma unroll
                             for (int q = 0; q < 4; ++q) {
@@ -302,7 +305,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                                     // share of the mirror row p[fs-1] = -p[fs+1]
                                     float M = 0.f;
 #pragma unroll
-                                    for (int kk = 0; kk < R; ++kk) M = __fmaf_rn(g.c[kk], at(wz[u + R - 2 + kk], q), M);
+                                    for (int kk = 0; kk < R; ++kk) M = __fmaf_rn(tap[kk], at(wz[u + R - 2 + kk], q), M);
                                     d -= M;
                                 }
                                 const int gx = gx0 + q;
@@ -376,14 +379,14 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                                 for (int t = 0; t < 3; ++t)
                                     f[t] = cpml_mix(lds4(sP + rr * RW + 4 * lane - 4 + 4 * t),
                                                     lds4(cp.bx[0] + 4 * lane + 4 * t), lds4(cp.ax[0] + 4 * lane + 4 * t), h[t]);
-                                grad_x4_of<R>(f[0], f[1], f[2], g.c, Dx);
+                                grad_x4_of<R>(f[0], f[1], f[2], tap, Dx);
                             } else {
-                                grad_x4<R>(sP + rr * RW, lane, g.c, Dx, mp1);
+                                grad_x4<R>(sP + rr * RW, lane, tap, Dx, mp1);
                             }
                         } else {
-                            grad_x4<R>(sP + rr * RW, lane, g.c, Dx, mp1);
+                            grad_x4<R>(sP + rr * RW, lane, tap, Dx, mp1);
                         }
-                        grad_z4<R>(wp, u, g.c, Dz);
+                        grad_z4<R>(wp, u, tap, Dz);
                         const float4 vx1 = lds4(sVX + rr * VXW + 4 * lane + 4);
                         const float4 vz1 = lds4(sVZ + (rv + 2 * R) * RW + 4 * lane);
                         const float4 a2 = lds4(sA2 + rv * RW + 4 * lane);
@@ -443,7 +446,7 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
                                         if (FS && gz == g.fs) {
                                             // the p update reads vz[fs-1] as vz[fs]
 #pragma unroll
-                                            for (int kk = 0; kk < R; ++kk) d = __fmaf_rn(g.c[kk], at(wp[u + R - 1 + kk], q), d);
+                                            for (int kk = 0; kk < R; ++kk) d = __fmaf_rn(tap[kk], at(wp[u + R - 1 + kk], q), d);
                                         }
                                         at(vz, q) = __fmaf_rn(at(a2, q), d, (1.f - at(k3, q)) * at(vz1, q));
                                         if (RHO) at(acc2[u], q) = __fmaf_rn(at(vz1, q), at(jzv, q), at(acc2[u], q));

@@ -59,7 +59,10 @@ fwd_batch_kernel(const int4 *__restrict__ items, const BatchModel *__restrict__ 
     const int4 item = items[blockIdx.x];   // (model, tile, group, 0)
     const BatchModel &M = models[item.x];
     const int t_end = mode == kBatchForward ? M.nt : min(M.nt, M.t_cache);
-    if (tau >= t_end) return;              // uniform per CTA
+    if (tau >= t_end) {                    // uniform per CTA
+        grid_dependency_wait();            // a launch ends after the one before it
+        return;
+    }
     const int par = mode == kBatchForward ? (tau & 1) : ((tau - t0) & 1);
     __shared__ FwdArgs A;
     if (threadIdx.x == 0) {
@@ -93,7 +96,10 @@ adj_batch_kernel(const int4 *__restrict__ items, const BatchModel *__restrict__ 
     if (clock) tau = *reinterpret_cast<const volatile int *>(clock) - tau;
     const int4 item = items[blockIdx.x];
     const BatchModel &M = models[item.x];
-    if (tau >= M.nt) return;
+    if (tau >= M.nt) {
+        grid_dependency_wait();
+        return;
+    }
     const int par = (M.nt - 1 - tau) & 1;
     __shared__ AdjArgs A;
     if (threadIdx.x == 0) {

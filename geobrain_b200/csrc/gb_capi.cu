@@ -945,6 +945,15 @@ int restore_checkpoint(gb_plan *P, float *state, const void *ckpts, int k, int f
     return GB_OK;
 }
 
+// Does a tile reach into the absorbing layers, the surface or the grid's edge?
+bool slow_tile(const gb_plan *P, int t)
+{
+    const int R = P->R, TZ = P->tz, nabc = P->d.nabc;
+    const int zlo = std::max(P->fs + 1, nabc), zhi = nabc + P->d.nz, xlo = nabc, xhi = nabc + P->d.nx;
+    const int z0 = (t / P->tiles_x) * TZ, x0 = (t % P->tiles_x) * TX;
+    return !(z0 - 2 * R >= zlo && z0 + TZ + 2 * R <= zhi && x0 - 8 >= xlo && x0 + TX + 8 <= xhi);
+}
+
 // The CTA schedule for `slots` resident CTAs of the tile kernels (every SM's
 // share).  Tiles whose rectangles reach into the absorbing frame, the free
 // surface or past the grid's edge take the masked, damped slow path: they go
@@ -957,16 +966,10 @@ void build_schedule(gb_plan *P, int slots)
                                         P->group_streams, P->d.n_shots, P->d.nabc, P->d.nz, P->d.nx, P->fs};
     if (key == P->sched_key) return;
     P->sched_key = key;
-    const int R = P->R, TZ = P->tz, nabc = P->d.nabc;
-    const int zlo = std::max(P->fs + 1, nabc), zhi = nabc + P->d.nz, xlo = nabc, xhi = nabc + P->d.nx;
-    auto slow = [&](int t) {
-        const int z0 = (t / P->tiles_x) * TZ, x0 = (t % P->tiles_x) * TX;
-        return !(z0 - 2 * R >= zlo && z0 + TZ + 2 * R <= zhi && x0 - 8 >= xlo && x0 + TX + 8 <= xhi);
-    };
     P->tile_order.clear();
     for (int pass = 0; pass < 2; ++pass)
         for (int t = 0; t < P->n_tiles; ++t)
-            if (slow(t) == (pass == 0)) P->tile_order.push_back(t);
+            if (slow_tile(P, t) == (pass == 0)) P->tile_order.push_back(t);
     P->sched_items.clear();
     P->sched_off.clear();
     P->sched_cnt.clear();
@@ -2218,36 +2221,6 @@ int check_batch(gb_plan *const *plans, int n, const gb_model_io *io, bool gradie
     return GB_OK;
 }
 
-int upload_batch(gb_plan *const *plans, int n, const std::vector<BatchModel> &models,
-                 const std::vector<BatchMaps> &maps, char *bws, const BatchLayout &B, cudaStream_t st)
-{
-    std::vector<int4> items;
-    items.reserve(B.n_items);
-    for (int m = 0; m < n; ++m)
-        for (int t = 0; t < plans[m]->n_tiles; ++t)
-            for (int g = 0; g < plans[m]->n_groups; ++g) items.push_back(int4{m, t, g, 0});
-    GB_CUDA(cudaMemcpyAsync(bws + B.models, models.data(), n * sizeof(BatchModel), cudaMemcpyHostToDevice, st));
-    GB_CUDA(cudaMemcpyAsync(bws + B.maps, maps.data(), n * sizeof(BatchMaps), cudaMemcpyHostToDevice, st));
-    GB_CUDA(cudaMemcpyAsync(bws + B.items, items.data(), items.size() * 16, cudaMemcpyHostToDevice, st));
-    return GB_OK;
-}
-
-int make_state_maps(const gb_plan *P, const float *buf, CUtensorMap (&m)[3])
-{
-    const int n_planes = 3 * P->d.n_shots;
-    if (int rc = make_map(&m[0], buf, P->Nx, P->Nz, P->pitch, n_planes, RW, box_rows_p(P->R, P->tz))) return rc;
-    if (int rc = make_map(&m[1], buf, P->Nx, P->Nz, P->pitch, n_planes, VXW, box_rows_p(P->R, P->tz))) return rc;
-    return make_map(&m[2], buf, P->Nx, P->Nz, P->pitch, n_planes, RW, box_rows_vz(P->R, P->tz));
-}
-
-int launch_batch(gb_plan *P0, const StepKernel &K, long long n_items, void **args, cudaStream_t st)
-{
-    GB_CUDA(launch_kernel(P0, K.fn, dim3((unsigned)n_items), dim3(NTHR), K.smem, args, st, false));
-    ++P0->launches;
-    ++P0->api_launches;
-    return GB_OK;
-}
-
 // The lanes of a batch: its models split into up to kBatchLanes runs of
 // consecutive models with about equal work items.  Inside a step graph each
 // lane's launches go to a stream of their own, so a lane starts its next
@@ -2280,6 +2253,44 @@ BatchLanes batch_lanes(gb_plan *const *plans, int n_models, long long n_items)
     L.cnt[lane] = acc - L.off[lane];
     L.n = lane + 1;
     return L;
+}
+
+// The items of a batch, lane by lane; in a lane those that take longest come
+// first, so that its launches end on short ones: most shots, then tiles on
+// the slow path.
+int upload_batch(gb_plan *const *plans, int n, const std::vector<BatchModel> &models,
+                 const std::vector<BatchMaps> &maps, char *bws, const BatchLayout &B, cudaStream_t st)
+{
+    std::vector<int4> items;
+    items.reserve(B.n_items);
+    for (int m = 0; m < n; ++m)
+        for (int t = 0; t < plans[m]->n_tiles; ++t)
+            for (int g = 0; g < plans[m]->n_groups; ++g) items.push_back(int4{m, t, g, 0});
+    const BatchLanes lanes = batch_lanes(plans, n, B.n_items);
+    auto cost = [&](const int4 &w) { return 2 * plans[w.x]->group_shots(w.z) + (slow_tile(plans[w.x], w.y) ? 1 : 0); };
+    for (int i = 0; i < lanes.n; ++i)
+        std::stable_sort(items.begin() + lanes.off[i], items.begin() + lanes.off[i] + lanes.cnt[i],
+                         [&](const int4 &a, const int4 &b) { return cost(a) > cost(b); });
+    GB_CUDA(cudaMemcpyAsync(bws + B.models, models.data(), n * sizeof(BatchModel), cudaMemcpyHostToDevice, st));
+    GB_CUDA(cudaMemcpyAsync(bws + B.maps, maps.data(), n * sizeof(BatchMaps), cudaMemcpyHostToDevice, st));
+    GB_CUDA(cudaMemcpyAsync(bws + B.items, items.data(), items.size() * 16, cudaMemcpyHostToDevice, st));
+    return GB_OK;
+}
+
+int make_state_maps(const gb_plan *P, const float *buf, CUtensorMap (&m)[3])
+{
+    const int n_planes = 3 * P->d.n_shots;
+    if (int rc = make_map(&m[0], buf, P->Nx, P->Nz, P->pitch, n_planes, RW, box_rows_p(P->R, P->tz))) return rc;
+    if (int rc = make_map(&m[1], buf, P->Nx, P->Nz, P->pitch, n_planes, VXW, box_rows_p(P->R, P->tz))) return rc;
+    return make_map(&m[2], buf, P->Nx, P->Nz, P->pitch, n_planes, RW, box_rows_vz(P->R, P->tz));
+}
+
+int launch_batch(gb_plan *P0, const StepKernel &K, long long n_items, void **args, cudaStream_t st)
+{
+    GB_CUDA(launch_kernel(P0, K.fn, dim3((unsigned)n_items), dim3(NTHR), K.smem, args, st, true));
+    ++P0->launches;
+    ++P0->api_launches;
+    return GB_OK;
 }
 
 // What the arguments of a batch's launches are made of: its workspace (with

@@ -244,6 +244,9 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
         for (int u = 0; u < G::LV; ++u) e_p[u] = e_vx[u] = e_vz[u] = zero4();
     }
 
+    // (a batch's arguments are in shared memory, where each barrier would have
+    // them read again)
+    const float tap[4] = {g.c[0], g.c[1], g.c[2], g.c[3]};
     for (int k = 0; k < ns; ++k) {
         const int s = s0 + k;
         const int b = k & 1;
@@ -306,7 +309,7 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                     const float4 a1 = lds4(sA1 + r * RW + 4 * lane);
                     const bool tile_cell = IMG >= 1 && r >= R && r < R + TZ && vlane;
                     if (fast) {
-                        divergence4<R>(sVX + r * VXW, lane, wz, u, g.c, D);
+                        divergence4<R>(sVX + r * VXW, lane, wz, u, tap, D);
 #pragma unroll
                         for (int q = 0; q < 4; ++q) at(pv, q) = __fmaf_rn(-at(a1, q), D[q], at(pv, q));
                         if (tile_cell && imaging)
@@ -326,7 +329,7 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                                 const long long po = (long long)s * 4 * g.plane + o;
                                 const float4 ox = d1[u], oz = e1[u];
                                 float Dx[4], Dz[4];
-                                divergence4_split<R>(sVX + r * VXW, lane, wz, u, g.c, Dx, Dz);
+                                divergence4_split<R>(sVX + r * VXW, lane, wz, u, tap, Dx, Dz);
                                 float4 nx = ox, nz = oz;
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
@@ -344,7 +347,7 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                                 if (lx) stg4(A.psi_out + po, nx);
                                 if (lz) stg4(A.psi_out + po + g.plane, nz);
                             } else {
-                                divergence4<R>(sVX + r * VXW, lane, wz, u, g.c, D);
+                                divergence4<R>(sVX + r * VXW, lane, wz, u, tap, D);
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
                                     const int gx = gx0 + q;
@@ -415,8 +418,8 @@ __device__ __forceinline__ void fwd_body(const CUtensorMap *mP, const CUtensorMa
                     if (fast || (gz < g.Nz && gx0 < g.Nx)) {
                         float Dx[4], Dz[4];
                         const float4 pv = wp[u + R - 1];        // p row rr
-                        grad_x4<R>(sP + rr * RW, lane, g.c, Dx, pv);
-                        grad_z4<R>(wp, u, g.c, Dz);
+                        grad_x4<R>(sP + rr * RW, lane, tap, Dx, pv);
+                        grad_z4<R>(wp, u, tap, Dz);
                         float4 vx = lds4(sVX + rr * VXW + 4 * lane + 4);
                         float4 vz = lds4(sVZ + (rv + 2 * R) * RW + 4 * lane);
                         const float4 a2 = lds4(sA2 + rv * RW + 4 * lane);

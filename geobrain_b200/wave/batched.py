@@ -72,8 +72,9 @@ class _Prepared:
             self.inputs.append((m["vp"], m["rho"], damp, w))
         for plan in self.plans:
             # up to 8 shots per CTA: fewer, longer CTAs measured faster than
-            # more, shorter ones even for small models
-            plan.set_tiling(BATCH_TILE_ROWS, min(plan.n_shots, 8))
+            # more, shorter ones even for small models; equal groups
+            groups = -(-plan.n_shots // 8)
+            plan.set_tiling(BATCH_TILE_ROWS, -(-plan.n_shots // groups))
         self.plan_arr = (ctypes.c_void_p * len(self.plans))(*[p.h.value for p in self.plans])
 
 
