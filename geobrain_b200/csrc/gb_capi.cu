@@ -430,6 +430,9 @@ struct gb_plan {
     // up but the last): 128 x 240, 40 shots, 300 steps 7.87 -> 7.33 (2 shots
     // per CTA for 1); 240 x 540, 12 shots, 200 steps 6.68 -> 5.60 (2 for 1);
     // 460 x 1260, 8 shots, 150 steps, CPML 25.3 -> 17.7 (4 + 4 for 7 + 1).
+    // A CPML step ends on its layer tiles, which take about twice an interior
+    // one's time: one or two groups leave these ends uncovered (8 shots as 3 +
+    // 3 + 2 15.6 ms, as 4 + 4 17.4; 16 as 6 + 6 + 4 18.8, as 8 + 8 21.3).
     int default_spc() const
     {
         const int S = d.n_shots;
@@ -440,7 +443,7 @@ struct gb_plan {
             if ((S + per - 1) / per != groups) continue;
             const double ctas = (double)n_tiles * groups;
             const double fill = ctas >= 592.0 ? 1.0 : ctas >= 296.0 ? std::pow(ctas / 592.0, 0.4) : 0.758 * ctas / 296.0;
-            const double cost = (0.82 * groups + S) / fill;
+            const double cost = (0.82 * groups + S) / fill * (cpml && groups < 3 ? 1.2 : 1.0);
             if (!best || cost < best_cost) best = per, best_cost = cost;
         }
         return std::max(1, best);
@@ -1364,7 +1367,7 @@ int gb_plan_set_absorbing(gb_plan *p, int mode, float vmax)
     if ((mode == GB_ABSORB_CPML) == p->cpml && (!p->cpml || vmax == p->cpml_vmax)) return GB_OK;   // unchanged
     p->release_graph();
     p->cpml = mode == GB_ABSORB_CPML;
-    p->res_choose();   // the resident forward runs the damping layers only
+    p->retile();   // other groups; the resident forward runs the damping layers only
     p->cpml_vmax = vmax;
     p->cpml_prof.clear();
     if (!p->cpml) return GB_OK;
