@@ -337,9 +337,8 @@ struct gb_plan {
     // where the per-step tile kernel is launch- and latency-bound), with the
     // two exchanges through global memory and the smallest tile height that
     // fits (the most CTAs).  At 8th order 4-row tiles are all boundary twice
-    // over (each row goes up and down: 140 x 240, 1000 steps 3.74 ms against
-    // 3.05 with 8 rows) and 12-row tiles with 8 warps are slower than 16 with
-    // 16 (3.77, 3.54): both are left out.  The cluster exchange (16 CTAs a shot at most)
+    // over (each row goes up and down: 140 x 240, 1000 steps 3.39 ms against
+    // 3.07 with 8 rows) and are left out.  The cluster exchange (16 CTAs a shot at most)
     // and one exchange a step (which sends twice the cells to eight
     // neighbours and updates p on twice the rows) measured no faster on the
     // 100 x 200 grid; they run when asked for.  More shots keep the tile
@@ -383,7 +382,7 @@ struct gb_plan {
                 const long long n = (long long)((Nx + TX - 1) / TX) * ((Nz + tz - 1) / tz);
                 if (cl && n > kMaxClusterTiles) continue;
                 if (res_mode < 0 && n * d.n_shots > sms) continue;
-                if (res_mode < 0 && !res_tz_req && R == 4 && (tz == 4 || tz == 12)) continue;
+                if (res_mode < 0 && !res_tz_req && R == 4 && tz == 4) continue;
                 best = tz;
                 res_cluster = cl;
                 res_single = sx;

@@ -79,7 +79,6 @@ struct ResGeo {
     static constexpr int LI = (NI + NW - 1) / NW;                    // interior rows per warp
     static constexpr int NB = TZ - NI;                               // boundary rows (all lanes)
     static constexpr int NITEM = NB * 30 + NI * 2;                   // boundary items of 4 cells
-    static constexpr int LE = (TZ + NW - 1) / NW;                    // energy rows per warp
     static constexpr size_t SMEM = size_t(3 * FL + NCOEF * CF) * 4;
 };
 
@@ -413,23 +412,46 @@ __device__ __forceinline__ const uint2 *res_halo(int h, float *rows_f, float *co
     return t < 0 ? nullptr : xb + ((size_t)t * kResParts + part) * G::PART + 4 * j;
 }
 
-// Receives the neighbours' boundary cells of one field pair into the halo,
-// polling each group's words for `tag`.  Uniform outcome.
+// The halo groups a thread receives each step, worked out once: the source
+// words of the p exchange (strips 0 .. 3; null where there is no neighbour;
+// the v exchange's are 4 strips on) and where they go.
 template <int R, int NW, int TZ>
-__device__ __forceinline__ bool res_receive(float *rows_f, float *cols_f, const uint2 *xb, const int (&nb)[4], int pb,
-                                            unsigned int tag, int *err)
-{
+struct ResRecv {
     using G = ResGeo<R, NW, TZ>;
-    bool ok = true;
-    for (int h = threadIdx.x; h < G::NHALO && ok; h += G::NTH) {
-        float *dst;
-        const uint2 *w = res_halo<R, NW, TZ>(h, rows_f, cols_f, xb, nb, pb, dst);
-        if (!w) continue;
-        float4 v;
-        ok = ll_get4(w, tag, v, err);
-        if (ok) sts4(dst, v);
+    static constexpr int NK = (G::NHALO + G::NTH - 1) / G::NTH;
+    const uint2 *w[NK];
+    float *dp[NK], *dv[NK];
+
+    __device__ __forceinline__ void init(float *sP, float *sVX, float *sVZ, const uint2 *xb, const int (&nb)[4])
+    {
+#pragma unroll
+        for (int k = 0; k < NK; ++k) {
+            const int h = threadIdx.x + k * G::NTH;
+            w[k] = h < G::NHALO ? res_halo<R, NW, TZ>(h, sP, sP, xb, nb, 0, dp[k]) : nullptr;
+            if (w[k]) res_halo<R, NW, TZ>(h, sVZ, sVX, xb, nb, 4, dv[k]);
+        }
     }
-    return __syncthreads_and(ok);
+    // Receives the neighbours' boundary cells of one field pair into the
+    // halo, polling each group's words for `tag`.  Uniform outcome.
+    template <bool V>
+    __device__ __forceinline__ bool get(unsigned int tag, int *err)
+    {
+        bool ok = true;
+#pragma unroll
+        for (int k = 0; k < NK; ++k)
+            if (ok && w[k]) {
+                float4 v;
+                ok = ll_get4(w[k] + (V ? 4 * G::PART : 0), tag, v, err);
+                if (ok) sts4(V ? dv[k] : dp[k], v);
+            }
+        return __syncthreads_and(ok);
+    }
+};
+
+__device__ __forceinline__ void add_square4(float4 &e, const float4 &v)
+{
+#pragma unroll
+    for (int q = 0; q < 4; ++q) at(e, q) = __fmaf_rn(at(v, q), at(v, q), at(e, q));
 }
 
 // The coefficients of the owned rows with the update masks and the damping
@@ -556,23 +578,21 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
     const bool ilane = lane >= 2 && lane <= 29;           // interior lanes
     const int ri = 2 * R + warp * G::LI;                  // first interior row of this warp
     const bool interior = G::NI > 0 && ilane && ri < TZ;  // this thread updates interior cells
-    // energy: bit 4u + q set where cell q of this lane's energy row u is summed
-    uint32_t emask = 0;
-    if (A.energy && lane >= 1 && lane <= 30) {
-        const int gx0 = x0 - 4 + 4 * lane;
+    // this thread's boundary item, and its halo groups
+    static_assert(G::NITEM <= G::NTH, "one boundary item per thread");
+    const bool item = threadIdx.x < G::NITEM;
+    int br = 0, bl = 0;
+    if (item) res_item<R, NW, TZ>(threadIdx.x, br, bl);
+    ResRecv<R, NW, TZ> recv;
+    if (!CL) recv.init(sP, sVX, sVZ, xb, K.nb);
+    // energy: the squares of the thread's own cells, LI interior groups and the
+    // item, added where the cells are computed (a pass of its own over the tile
+    // took 12 shared-memory reads a thread and a barrier a step).  Cells off
+    // the interior are summed too: the maps' readers take the interior only.
+    const bool energy = A.energy != 0;
+    float4 e_p[G::LI + 1], e_vx[G::LI + 1], e_vz[G::LI + 1];
 #pragma unroll
-        for (int u = 0; u < G::LE; ++u) {
-            const int r = R + warp + NW * u;
-            const int gz = z0 - R + r;
-            if (r < R + TZ && gz >= g.pml && gz < g.pml + g.nz && gz < g.Nz && gx0 < g.Nx)
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (gx0 + q >= g.pml && gx0 + q < g.pml + g.nx) emask |= 1u << (4 * u + q);
-        }
-    }
-    float4 e_p[G::LE], e_vx[G::LE], e_vz[G::LE];
-#pragma unroll
-    for (int u = 0; u < G::LE; ++u) e_p[u] = e_vx[u] = e_vz[u] = zero4();
+    for (int u = 0; u < G::LI + 1; ++u) e_p[u] = e_vx[u] = e_vz[u] = zero4();
     __syncthreads();
     if (CL) cluster_arrive();   // the first step's v exchange waits on this phase
 
@@ -585,21 +605,23 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
             for (int t = 0; t < G::LI + 2 * R - 1; ++t) wz[t] = lds4(sVZ + (ri - R + t) * RS + 4 * lane);
 #pragma unroll
             for (int u = 0; u < G::LI; ++u)
-                if (ri + u < TZ) res_p_cells<R, IMG>(A, C, ri + u, lane, wz, u, it, img);
+                if (ri + u < TZ) {
+                    const float4 pv = res_p_cells<R, IMG>(A, C, ri + u, lane, wz, u, it, img);
+                    if (energy) add_square4(e_p[u], pv);
+                }
         }
         // ---- the neighbours' v boundary cells of the previous step ---------
         // (a mirror row arrives mirrored: its owner sends it after the mirror)
         if (CL) cluster_wait();
-        else if (it > A.it0 && !res_receive<R, NW, TZ>(sVZ, sVX, xb, K.nb, 4, tag_v(it - 1), A.err)) return;
+        else if (it > A.it0 && !recv.template get<true>(tag_v(it - 1), A.err)) return;
         // ---- p boundary (sent on as computed), mirror ----------------------
-        for (int i = threadIdx.x; i < G::NITEM; i += G::NTH) {
-            int r, l;
-            res_item<R, NW, TZ>(i, r, l);
+        if (item) {
             float4 wz[2 * R];
 #pragma unroll
-            for (int t = 0; t < 2 * R; ++t) wz[t] = lds4(sVZ + (r - R + t) * RS + 4 * l);
-            const float4 pv = res_p_cells<R, IMG>(A, C, r, l, wz, 0, it, img);
-            if (!(fs_own && r == rm)) res_send4<R, TZ, CL>(K, K.rP, 0, 2, true, true, r, l, pv, tag_p(it));
+            for (int t = 0; t < 2 * R; ++t) wz[t] = lds4(sVZ + (br - R + t) * RS + 4 * bl);
+            const float4 pv = res_p_cells<R, IMG>(A, C, br, bl, wz, 0, it, img);
+            if (!(fs_own && br == rm)) res_send4<R, TZ, CL>(K, K.rP, 0, 2, true, true, br, bl, pv, tag_p(it));
+            if (energy) add_square4(e_p[G::LI], pv);
         }
         __syncthreads();
         if (fs_own) {
@@ -623,25 +645,25 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
                 if (ri + u < TZ) {
                     float4 vx, vz;
                     res_v_cells<R, IMG>(A, C, ri + u, lane, wp, u, vx, vz, img);
+                    if (energy) add_square4(e_vx[u], vx), add_square4(e_vz[u], vz);
                 }
         }
         // ---- the neighbours' p boundary cells ------------------------------
         if (CL) cluster_wait();
-        else if (!res_receive<R, NW, TZ>(sP, sP, xb, K.nb, 0, tag_p(it), A.err)) return;
+        else if (!recv.template get<false>(tag_p(it), A.err)) return;
         // ---- v boundary (sent on unless this is the launch's last step), mirror
         const bool send_v = it + 1 < A.it1;
-        for (int i = threadIdx.x; i < G::NITEM; i += G::NTH) {
-            int r, l;
-            res_item<R, NW, TZ>(i, r, l);
+        if (item) {
             float4 wp[2 * R];
 #pragma unroll
-            for (int t = 0; t < 2 * R; ++t) wp[t] = lds4(sP + (r - R + 1 + t) * RS + 4 * l);
+            for (int t = 0; t < 2 * R; ++t) wp[t] = lds4(sP + (br - R + 1 + t) * RS + 4 * bl);
             float4 vx, vz;
-            res_v_cells<R, IMG>(A, C, r, l, wp, 0, vx, vz, img);
+            res_v_cells<R, IMG>(A, C, br, bl, wp, 0, vx, vz, img);
             if (send_v) {
-                res_send4<R, TZ, CL>(K, K.rVZ, 4, 6, !(fs_own && r == rm), false, r, l, vz, tag_v(it));
-                res_send4<R, TZ, CL>(K, K.rVX, 4, 6, false, true, r, l, vx, tag_v(it));
+                res_send4<R, TZ, CL>(K, K.rVZ, 4, 6, !(fs_own && br == rm), false, br, bl, vz, tag_v(it));
+                res_send4<R, TZ, CL>(K, K.rVX, 4, 6, false, true, br, bl, vx, tag_v(it));
             }
+            if (energy) add_square4(e_vx[G::LI], vx), add_square4(e_vz[G::LI], vz);
         }
         __syncthreads();
         if (fs_own) {
@@ -653,7 +675,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
             }
             __syncthreads();
         }
-        // ---- receivers of this tile (acoustic_2d.py:272-274), energy -------
+        // ---- receivers of this tile (acoustic_2d.py:272-274) ---------------
         if (has_rcv) {
             for (int e = rcv0 + threadIdx.x; e < rcv1; e += G::NTH) {
                 const int4 en = A.rcv_ent[e];
@@ -663,26 +685,8 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
                 if (A.tr_vx) A.tr_vx[t] = sVX[o];
                 if (A.tr_vz) A.tr_vz[t] = sVZ[o];
             }
+            __syncthreads();   // the next step writes p, which the receivers read
         }
-        if (emask) {
-#pragma unroll
-            for (int u = 0; u < G::LE; ++u) {
-                if (((emask >> (4 * u)) & 15u) == 0) continue;
-                const int r = R + warp + NW * u;
-                const float4 pv = lds4(sP + r * RS + 4 * lane), vx = lds4(sVX + r * RS + 4 * lane);
-                const float4 vz = lds4(sVZ + r * RS + 4 * lane);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if ((emask >> (4 * u + q)) & 1u) {
-                        at(e_p[u], q) = __fmaf_rn(at(pv, q), at(pv, q), at(e_p[u], q));
-                        at(e_vx[u], q) = __fmaf_rn(at(vx, q), at(vx, q), at(e_vx[u], q));
-                        at(e_vz[u], q) = __fmaf_rn(at(vz, q), at(vz, q), at(e_vz[u], q));
-                    }
-                }
-            }
-        }
-        // the next step writes p, which the receivers and the energy sums read
-        __syncthreads();
         if (CL) cluster_arrive();
     }
     // the neighbours may still be sending into this CTA's halo: none leaves
@@ -701,13 +705,13 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_fwd_kernel(const ResArgs 
             stg4(st + 2 * g.plane + o, lds4(sVZ + (R + r) * RS + 4 * l));
         }
     }
-    if (A.energy && lane >= 1 && lane <= 30) {
-        const int gx0 = x0 - 4 + 4 * lane;
+    if (energy) {
 #pragma unroll
-        for (int u = 0; u < G::LE; ++u) {
-            const int gz = z0 + warp + NW * u;
-            if (warp + NW * u < TZ && gz >= g.pml && gz < g.pml + g.nz && gx0 < g.Nx) {
-                const long long o = (long long)gz * g.pitch + gx0;
+        for (int u = 0; u < G::LI + 1; ++u) {
+            const bool mine = u < G::LI ? interior && ri + u < TZ : item;
+            const int gz = z0 - R + (u < G::LI ? ri + u : br), gx = x0 - 4 + 4 * (u < G::LI ? lane : bl);
+            if (mine && gz >= g.pml && gz < g.pml + g.nz && gx < g.Nx) {
+                const long long o = (long long)gz * g.pitch + gx;
                 red_add_v4(A.energy_map + o, e_p[u]);
                 red_add_v4(A.energy_map + g.plane + o, e_vx[u]);
                 red_add_v4(A.energy_map + 2 * g.plane + o, e_vz[u]);

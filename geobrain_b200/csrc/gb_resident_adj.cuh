@@ -170,6 +170,8 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_adj_kernel(const ResArgs 
     const bool item = threadIdx.x < G::NITEM;
     int br = 0, bl = 0;
     if (item) res_item<R, NW, TZ>(threadIdx.x, br, bl);
+    ResRecv<R, NW, TZ> recv;
+    recv.init(sP, sVX, sVZ, xb, K.nb);
     int off[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_adj_kernel(const ResArgs 
                 if (ri + u < TZ) sum_p(u, res_mu_p<R>(A, C, sQ, ri + u, lane, wz, u));
         }
         // ---- the neighbours' mu_v boundary cells of the previous step --------
-        if (n > 0 && !res_receive<R, NW, TZ>(sVZ, sVX, xb, K.nb, 4, tag_v(n - 1), A.err)) return;
+        if (n > 0 && !recv.template get<true>(tag_v(n - 1), A.err)) return;
         // ---- mu_p boundary (sent on as computed) ----------------------------
         if (item) {
             float4 wz[2 * R];
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_adj_kernel(const ResArgs 
                 }
         }
         // ---- the neighbours' mu_p boundary cells -----------------------------
-        if (!res_receive<R, NW, TZ>(sP, sP, xb, K.nb, 0, tag_p(n), A.err)) return;
+        if (!recv.template get<false>(tag_p(n), A.err)) return;
         // ---- mu_v boundary (sent on unless this is the last step) -------------
         if (item) {
             float4 wp[2 * R];
