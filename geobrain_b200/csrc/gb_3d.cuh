@@ -201,13 +201,17 @@ __global__ void mirror3_kernel(const Geo3 g, float *state, int field, int from, 
     }
 }
 
-// vx, vy, vz updates and their energy sums (same blocks as p3_kernel)
+// vx, vy, vz updates and their energy sums (same blocks as p3_kernel).  The
+// planes run down where p3_kernel's run up, so that each kernel starts on
+// planes the one before left in L2: 200^3, 4 shots, 30 steps 18.5 -> 18.2 ms,
+// and with adj_v3_kernel the other way from adj_p3_kernel a 130 x 149 x 171
+// gradient of 40 steps 24.4 -> 23.9.
 __global__ void __launch_bounds__(128, 7) v3_kernel(const Args3 A)
 {
     const Geo3 &g = A.g;
     const int x0 = 4 * (blockIdx.x * 32 + threadIdx.x);
     const int y = blockIdx.y * 4 + threadIdx.y;
-    const int z = blockIdx.z;
+    const int z = g.Nz - 1 - blockIdx.z;
     if (x0 >= g.Nx || y >= g.Ny) return;
     const long long o = (long long)z * g.plane + (long long)y * g.pitch + x0;
     const bool zin = z >= g.fs && z < g.Nz - 1;
@@ -426,7 +430,7 @@ __global__ void __launch_bounds__(128, RHO ? 4 : 5) adj_v3_kernel(const AdjArgs3
     const Geo3 &g = A.g;
     const int x0 = 4 * (blockIdx.x * 32 + threadIdx.x);
     const int y = blockIdx.y * 4 + threadIdx.y;
-    const int z = blockIdx.z;
+    const int z = g.Nz - 1 - blockIdx.z;
     if (x0 >= g.Nx - 1 || y < 1 || y >= g.Ny - 1 || z < g.fs || z >= g.Nz - 1) return;
     const long long o = (long long)z * g.plane + (long long)y * g.pitch + x0;
     const bool vy_row = y < g.Ny - 2, vz_row = z < g.Nz - 2;
