@@ -418,31 +418,33 @@ struct gb_plan {
         return n;
     }
 
-    // Shots per CTA: the S shots go to g groups of about equal size, at most 8
+    // Shots per CTA: the S shots go to g groups of about equal size, at most 16
     // shots each.  A CTA costs its shots and about 0.82 of a shot (its
     // coefficient tiles, and the energy or gradient partial sums that each
-    // group adds at each step), so fewer groups are less work; and a step of
+    // group adds at each step), so fewer groups are less work.  But a step of
     // tiles x g CTAs fills the 296 resident slots only when there are more of
-    // them, as the groups' streams cover each other's ends: measured, 0.5 of
-    // the rate at 160 CTAs, 0.75 at 300, 0.89 at 450, 1 from 592 on.
-    // Gradient, ms, against the fewest groups that give 592 CTAs (all filled
-    // up but the last): 128 x 240, 40 shots, 300 steps 7.87 -> 7.33 (2 shots
-    // per CTA for 1); 240 x 540, 12 shots, 200 steps 6.68 -> 5.60 (2 for 1);
-    // 460 x 1260, 8 shots, 150 steps, CPML 25.3 -> 17.7 (4 + 4 for 7 + 1).
-    // A CPML step ends on its layer tiles, which take about twice an interior
-    // one's time: one or two groups leave these ends uncovered (8 shots as 3 +
-    // 3 + 2 15.6 ms, as 4 + 4 17.4; 16 as 6 + 6 + 4 18.8, as 8 + 8 21.3).
+    // them (measured, 0.5 of the rate at 160 CTAs, 0.75 at 300, 0.89 at 450, 1
+    // from 592 on), and one group has no other beside it while its launches
+    // end and start: a tenth slower, two groups 3 %.  With CPML the ends are
+    // layer tiles, which take about twice an interior one's time: 1.2 more.
+    // Gradient, ms, each against the choice before it:
+    //   128 x 240, 40 shots, 300 steps: 2 a CTA 7.33, 1 a CTA 7.87
+    //   240 x 540, 12 shots, 200 steps: 2 a CTA 5.60, 1 a CTA 6.68
+    //   460 x 1260, 32 shots, 160 steps: 11 a CTA 38.2, 8 a CTA 39.1
+    //   1080 x 3080, 16 shots, recompute: 8 a CTA 61.8, 16 a CTA 65.7
+    //   460 x 1260, 8 shots, CPML: 3 + 3 + 2 15.6, 4 + 4 17.4, 7 + 1 25.3
     int default_spc() const
     {
         const int S = d.n_shots;
         int best = 0;
         double best_cost = 0.0;
-        for (int groups = (S + 7) / 8; groups <= S; ++groups) {
+        for (int groups = (S + 15) / 16; groups <= S; ++groups) {
             const int per = (S + groups - 1) / groups;
             if ((S + per - 1) / per != groups) continue;
             const double ctas = (double)n_tiles * groups;
             const double fill = ctas >= 592.0 ? 1.0 : ctas >= 296.0 ? std::pow(ctas / 592.0, 0.4) : 0.758 * ctas / 296.0;
-            const double cost = (0.82 * groups + S) / fill * (cpml && groups < 3 ? 1.2 : 1.0);
+            double cost = (0.82 * groups + S) / fill;
+            if (groups < 3) cost *= (groups == 1 ? 1.1 : 1.03) * (cpml ? 1.2 : 1.0);
             if (!best || cost < best_cost) best = per, best_cost = cost;
         }
         return std::max(1, best);
