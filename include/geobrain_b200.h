@@ -103,20 +103,22 @@ int gb_plan_create(const gb_model_desc *desc,
 void gb_plan_destroy(gb_plan *plan);
 
 /* Tile height (rows per CTA, 16 or 32) and shots per CTA; 0 keeps the
- * default.  Used by the autotuner. */
+ * default, which weighs what each group of shots costs against unfilled
+ * SMs (gb_plan_get_config tells).  Used by the autotuner. */
 int gb_plan_set_tiling(gb_plan *plan, int tile_rows, int shots_per_cta);
 
 /* Plain forward (gb_forward without a gradient store) as replays of one
  * CUDA graph of `steps` time steps (even, at most 64; 0 = one launch per
  * step and group; 16 by default).  The same chunk length drives the graphs
  * of the gradient (the forward steps that keep their imaging fields and the
- * adjoint steps over them) and of the batched forward and adjoint; each of
- * those graphs is captured on the first call and kept while the buffers are
- * the same.  The graph holds the step kernels of every shot group,
- * with their fork and join, and a step-counter update.  It is captured on
- * the first call, kept on the plan and replayed nt / steps times; the
- * remaining steps launch one by one.  A call with other buffers (workspace,
- * wavelet or trace pointers) captures it again. */
+ * adjoint steps over them) and of the batched forward and adjoint.  A graph
+ * holds the step kernels of every shot group, with their fork and join, and
+ * a step-counter update.  It is captured on the first call, kept on the plan
+ * and replayed nt / steps times; the remaining steps launch one by one.  A
+ * call with other buffers (workspace, wavelet or trace pointers) replaces
+ * the kernels' arguments in the kept graph.  With 0, a gradient is plain
+ * launches only: no graph, and no cooperative launch of the resident
+ * kernels. */
 int gb_plan_set_graph_steps(gb_plan *plan, int steps);
 
 /* Order of the tile kernels' CTAs in a time step.  mode 0 (default):
@@ -185,8 +187,10 @@ int gb_plan_autotune(gb_plan *plan, const float *vp, const float *rho, const flo
                      const float *wavelet, void *workspace, size_t workspace_bytes, int32_t steps,
                      void *stream, float *best_ms_per_step);
 
-/* Resident forward (plain gb_forward without a store, damping layers only):
- * one launch runs many time steps, each CTA keeping a 120-column x
+/* Resident kernels (damping layers only): the plain forward, and with modes
+ * -1 and 1 the gradient of a store that keeps every step's imaging fields
+ * (its adjoint when the residuals are of the pressure alone and every shot
+ * is a group of its own): one launch runs many time steps, each CTA keeping a 120-column x
  * tile_rows tile of one shot, plus its halo, in shared memory.  The thread
  * that updates a cell next to a tile edge sends it to the neighbouring
  * tile, and the rest of the tile is updated while it travels.
@@ -195,7 +199,7 @@ int gb_plan_autotune(gb_plan *plan, const float *vp, const float *rho, const flo
  * bit for bit.  mode: -1 automatic (the default: on when every shot's tiles
  * fit on the device's SMs at once, one CTA per SM, with the exchange through
  * global memory after each half-step and the smallest tile height that
- * fits), 0 off, 1 on with the exchange
+ * fits; 8 rows at least at 8th order), 0 off, 1 on with the exchange
  * through global memory (a cooperative launch; each float travels as an
  * 8-byte (value, tag) word the receiver polls, bounded; shots beyond one
  * launch run in further launches), 2 on with the exchange through
@@ -217,8 +221,8 @@ int gb_plan_set_resident(gb_plan *plan, int mode, int tile_rows);
  * global memory.  Any pointer may be NULL. */
 int gb_plan_get_resident(const gb_plan *plan, int *tile_rows, int *shots_per_launch, int *cluster);
 
-/* Run each group of shots on its own stream (forked from and joined back to
- * the caller's stream; on by default).  Groups never interact, so their
+/* Run the groups of shots on up to four streams (forked from and joined back
+ * to the caller's stream; on by default).  Groups never interact, so their
  * kernels fill each other's tails. */
 int gb_plan_set_group_streams(gb_plan *plan, int enable);
 
