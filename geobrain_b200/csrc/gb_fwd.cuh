@@ -94,7 +94,8 @@ __device__ __forceinline__ void stage_loads(const CUtensorMap *mP, const CUtenso
 // before all have come for shot k (the barrier in the middle of a shot), so
 // one counter does.
 // (A refill by thread 0 after the next shot's middle barrier left a load half
-// a shot's time, about 1.5 us, to arrive.)
+// a shot's time, about 1.5 us, to arrive: a step of 32 shots of 464 x 1320 took
+// 110 us at 4th order and 120 at 8th, against 103 and 115.)
 __device__ __forceinline__ bool last_warp_of_shot(unsigned *done, int lane)
 {
     static_assert((NWARP & (NWARP - 1)) == 0, "the counter's low bits count one shot's warps");

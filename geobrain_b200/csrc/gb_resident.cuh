@@ -22,7 +22,8 @@
 //   p interior;  receive the neighbours' v boundary cells of the previous
 //   step into the halo;  p boundary (sending each cell on), source,
 //   free-surface mirror;  v interior;  receive the p boundary cells;
-//   v boundary (sending on), mirror;  receivers and energy,
+//   v boundary (sending on), mirror;  receivers (the energy sums are added
+//   as the cells are computed),
 //
 // and the time a boundary cell takes to reach the neighbours is spent on
 // interior work.  The cell arithmetic is the tile kernel's, tap for tap (the
