@@ -512,8 +512,11 @@ __global__ void __launch_bounds__(128, RHO ? 4 : 5) adj_v3_kernel(const AdjArgs3
 // pressure injection (lam_p is then the adjoint of p just after the source was
 // added, acoustic_3d.py:153-163).  The state keeps lam_p on the p mask only;
 // for a source off it, lam_p is the running sum of what reaches the cell: the
-// receivers in it and the divergence of mu_v, kept in off[s].  A source in
-// the mirror plane is overwritten by the mirror: zero.
+// receivers in it and the divergence of mu_v, kept in off[s].  In plane fs + 1
+// under a free surface the cell is read a second time, as the mirror cell
+// p[fs-1] = -p[fs+1]: minus the receivers in that one and minus its share of
+// the divergence, c2 mu_vz[fs] (all else there is zero).  A source in the
+// mirror plane is overwritten by the mirror: zero.
 __global__ void wavelet_grad3_kernel(const AdjArgs3 A, const int *src, const int *rcv, const float *res_p,
                                      float *grad_wavelet, float *off, int it)
 {
@@ -534,14 +537,19 @@ __global__ void wavelet_grad3_kernel(const AdjArgs3 A, const int *src, const int
                        ? 0.f
                        : P[(long long)f * g.vol + (long long)zz * g.plane + (long long)yy * g.pitch + xx];
         };
+        const bool mirrored = A.free_surface && z == g.fs + 1;
         lam = off[s];
         if (res_p)
             for (int r = 0; r < g.n_rcv; ++r)
-                if (rcv[r] == z && rcv[g.n_rcv + r] == y && rcv[2 * g.n_rcv + r] == x)
-                    lam += res_p[((long long)s * g.nt + it) * g.n_rcv + r];
+                if (rcv[g.n_rcv + r] == y && rcv[2 * g.n_rcv + r] == x) {
+                    const float v = res_p[((long long)s * g.nt + it) * g.n_rcv + r];
+                    if (rcv[r] == z) lam += v;
+                    if (mirrored && rcv[r] == g.fs - 1) lam -= v;
+                }
         lam += d4f(at(1, z, y, x), at(1, z, y, x - 1), at(1, z, y, x + 1), at(1, z, y, x - 2)) +
                d4f(at(2, z, y, x), at(2, z, y - 1, x), at(2, z, y + 1, x), at(2, z, y - 2, x)) +
                d4f(at(3, z, y, x), at(3, z - 1, y, x), at(3, z + 1, y, x), at(3, z - 2, y, x));
+        if (mirrored) lam -= kC2 * at(3, g.fs, y, x);
         off[s] = lam;
     }
     grad_wavelet[(long long)s * g.nt + it] = g.dt * lam;

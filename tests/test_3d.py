@@ -375,3 +375,35 @@ def test_cuda_3d_gradients_at_the_rims(cuda_device, free_surface):
     assert orc.rel_l2(r.grad.cpu().numpy(), gr) < 1e-4
     for i in range(4):
         assert orc.rel_l2(s.grad[i].cpu().numpy(), gw[i]) < 1e-4, i
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fields", [("p",), ("p", "vx", "vy", "vz")])
+def test_cuda_3d_wavelet_gradient_of_border_sources_below_the_surface(cuda_device, fields):
+    """Sources off the pressure mask in the plane that the free surface
+    mirrors (fs + 1): p there is read again, with its sign turned, by vz of
+    plane fs and by receivers in the mirror plane of that column.  Three such
+    columns and one on the mask, each with a receiver in the mirror plane, the
+    first also with one in the source's cell, against the float64 oracle, 1e-4 as above."""
+    from geobrain_b200.wave import acoustic_forward_kernel_3d, bc_pml_3d
+    rng = np.random.default_rng(23)
+    nz, ny, nx, nabc, nt = 13, 14, 37, 6, 44
+    vp = (2000 + 800 * rng.random((nz, ny, nx))).astype(np.float32)
+    rho = (1900 + 300 * rng.random((nz, ny, nx))).astype(np.float32)
+    damp = bc_pml_3d(nx, ny, nz, 10.0, 10.0, 10.0, nabc, float(vp.max()), free_surface=False).astype(np.float32)
+    w = rng.standard_normal((4, nt)).astype(np.float32)
+    sx, sy = np.array([4, 1 - nabc, nx + nabc - 2, 30]), np.array([1 - nabc, 5, 7, 9])
+    src = dict(src_x=sx, src_y=sy, src_z=np.ones(4, np.int64), src_v=w)
+    rcv = dict(rcv_x=np.append(sx, [4, 10]), rcv_y=np.append(sy, [1 - nabc, 5]), rcv_z=np.array([-1, -1, -1, -1, 1, 3]))
+    kw = dict(nz=nz, ny=ny, nx=nx, nt=nt, dt=1e-3, nabc=nabc, free_surface=True, **rcv)
+    res = {k: rng.standard_normal((4, nt, 6)).astype(np.float32) for k in fields}
+    t = lambda a: torch.as_tensor(a, device=cuda_device)
+    v, s = (t(a).requires_grad_(True) for a in (vp, w))
+    out = acoustic_forward_kernel_3d(dx=10.0, dy=10.0, dz=10.0, src_n=4, rcv_n=6, damp=t(damp), vp=v, rho=t(rho),
+                                     device=cuda_device, **kw, **dict(src, src_v=s))
+    sum((t(res[k]) * out[k]).sum() for k in res).backward()
+    gv, _, gw = o3.gradient(dz=10.0, damp=damp, vp=vp, rho=rho, with_wavelet=True, **kw, **src,
+                            **{f"res_{k}": x for k, x in res.items()})
+    assert orc.rel_l2(v.grad.cpu().numpy(), gv) < 1e-4
+    for i in range(4):
+        assert orc.rel_l2(s.grad[i].cpu().numpy(), gw[i]) < 1e-4, i
