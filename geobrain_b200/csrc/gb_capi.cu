@@ -175,8 +175,8 @@ struct gb_plan {
     // that keep their imaging fields, the adjoint steps over them, and the
     // batched forward / adjoint steps (on a batch's first plan).  `key` is
     // what a graph's shape depends on (device, kernel, steps, streams), `args`
-    // what its kernels' arguments were made of: with other arguments (another
-    // workspace, other traces) its nodes get new parameters, in order, in
+    // its kernels' arguments (arg_words): with others (another workspace or
+    // layout in it, other traces) its nodes get new parameters, in order, in
     // place of a new capture (which took 12 ms of host time for 64 launches
     // and waited for the device).
     struct GraphSlot {
@@ -788,6 +788,22 @@ inline void lane_shots(const gb_plan *P, int g0, int gc, int *s0, int *ns)
     *ns = std::min(P->d.n_shots, P->group_first(g0 + gc)) - *s0;
 }
 
+// The bytes of a chunk's kernel arguments, for GraphSlot::args: the maps, the
+// argument struct and the pointers that vary from step to step, as they are
+// passed, so that nothing they were made of can be left out.
+template <class... T>
+std::vector<uintptr_t> arg_words(const T &...parts)
+{
+    std::vector<uintptr_t> w;
+    auto add = [&](const void *p, size_t bytes) {
+        const size_t at = w.size();
+        w.resize(at + (bytes + sizeof(uintptr_t) - 1) / sizeof(uintptr_t), 0);
+        std::memcpy(w.data() + at, p, bytes);
+    };
+    (add(&parts, sizeof(parts)), ...);
+    return w;
+}
+
 // ---------------------------------------------------------------------------
 // CUDA graphs of chunks of steps.  A graph holds C steps of every lane (C
 // even, so step j of the chunk reads state level j & 1) with the lanes' fork
@@ -1315,6 +1331,7 @@ int gb_plan_set_resident(gb_plan *p, int mode, int tile_rows)
     bool known = tile_rows == 0;
     for (int tz : kResidentRows) known |= tz == tile_rows;
     if (!known) return fail(GB_E_ARG, "tile_rows must be 0, 4, 8, 12, 16, 24, 32, 36 or 40");
+    p->release_graph();   // the layout of the workspaces follows the tiling
     p->res_mode = mode;
     p->res_tz_req = tile_rows;
     p->res_choose();
@@ -1527,7 +1544,7 @@ int gb_forward(gb_plan *P, const float *vp, const float *rho, const float *damp,
     if (int rc = prepare_kernel(K0)) return rc;
     if (store && store->cached_steps > 0)
         if (int rc = prepare_kernel(KI)) return rc;
-    Maps maps[2];
+    Maps maps[2]{};
     for (int b = 0; b < 2; ++b)
         if (int rc = make_maps(P, buf[b], Su.a1, Su.a2, &maps[b])) return rc;
 
@@ -1562,12 +1579,9 @@ int gb_forward(gb_plan *P, const float *vp, const float *rho, const float *damp,
         int dev = -1;
         GB_CUDA(cudaGetDevice(&dev));
         const std::vector<uintptr_t> key = {(uintptr_t)dev, (uintptr_t)K0.fn, (uintptr_t)C, (uintptr_t)gs.n};
-        const std::vector<uintptr_t> args = {
-            (uintptr_t)ws, (uintptr_t)wavelet, (uintptr_t)trace_p, (uintptr_t)trace_vx, (uintptr_t)trace_vz,
-            (uintptr_t)want_energy, (uintptr_t)P->tz, (uintptr_t)P->spc_eff, (uintptr_t)P->n_groups,
-            (uintptr_t)P->sched, (uintptr_t)d.nt};
         FwdArgs B = A;
         B.step_base = step_ctr;
+        const std::vector<uintptr_t> args = arg_words(maps, B, buf, Su.psi, P->d_items);
         if (int rc = capture_chunk(P, P->g_fwd, key, args, C, step_ctr, C, true, [&](int j, const GroupStreams &g) {
                 FwdArgs Bj = B;
                 Bj.it = j;
@@ -1647,17 +1661,16 @@ int gb_forward(gb_plan *P, const float *vp, const float *rho, const float *damp,
             int dev = -1;
             GB_CUDA(cudaGetDevice(&dev));
             const std::vector<uintptr_t> key = {(uintptr_t)dev, (uintptr_t)KI.fn, (uintptr_t)C, (uintptr_t)gs.n};
-            const std::vector<uintptr_t> args = {
-                (uintptr_t)ws, (uintptr_t)wavelet, (uintptr_t)trace_p, (uintptr_t)trace_vx, (uintptr_t)trace_vz,
-                (uintptr_t)want_energy, (uintptr_t)P->tz, (uintptr_t)P->spc_eff, (uintptr_t)P->n_groups,
-                (uintptr_t)store->imaging, (uintptr_t)t_cache, (uintptr_t)store->imaging_format,
-                (uintptr_t)store->with_rho, (uintptr_t)P->sched, (uintptr_t)d.nt};
             FwdArgs B = A;
+            B.it = 0;                       // these, and imaging below, each step sets anew
+            B.out = B.psi_out = nullptr;
+            B.psi_in = nullptr;
             B.step_base = step_ctr;
             B.img_base = reinterpret_cast<float *>(store->imaging);
             B.img_step = (long long)step_img;
             B.img_t0 = t_cache;
             B.imaging = reinterpret_cast<float *>(store->imaging);
+            const std::vector<uintptr_t> args = arg_words(maps, B, buf, Su.psi, P->d_items);
             if (int rc = capture_chunk(P, P->g_fwd_img, key, args, C, step_ctr, C, true, [&](int j, const GroupStreams &g) {
                     FwdArgs Bj = B;
                     Bj.it = j;
@@ -1942,7 +1955,7 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
     const StepKernel KA = adj_kernel(P->R, P->tz, fs, rho_fields, ifmt, P->cpml);
     if (int rc = prepare_kernel(KF)) return rc;
     if (int rc = prepare_kernel(KA)) return rc;
-    Maps fmaps[2], amaps[2];
+    Maps fmaps[2]{}, amaps[2]{};
     for (int b = 0; b < 2; ++b) {
         if (int rc = make_maps(P, fb[b], Su.a1, Su.a2, &fmaps[b])) return rc;
         if (int rc = make_maps(P, mu[b], Su.a1, Su.a2, &amaps[b])) return rc;
@@ -2013,17 +2026,17 @@ int gb_backward(gb_plan *P, const float *vp, const float *rho, const float *damp
                 int dev = -1;
                 GB_CUDA(cudaGetDevice(&dev));
                 const std::vector<uintptr_t> key = {(uintptr_t)dev, (uintptr_t)KA.fn, (uintptr_t)C, (uintptr_t)gs.n};
-                const std::vector<uintptr_t> args = {
-                    (uintptr_t)ws, (uintptr_t)res_p, (uintptr_t)res_vx, (uintptr_t)res_vz, (uintptr_t)img_base,
-                    (uintptr_t)img_fmt, (uintptr_t)t0, (uintptr_t)grad_wavelet, (uintptr_t)P->tz,
-                    (uintptr_t)P->spc_eff, (uintptr_t)P->n_groups, (uintptr_t)rho_fields, (uintptr_t)P->sched,
-                    (uintptr_t)d.nt};
                 AdjArgs B = A;
+                B.it = 0;                   // these, each step sets anew
+                B.out = B.eta_out = nullptr;
+                B.img = nullptr;
+                B.eta_in = nullptr;
                 B.step_base = step_ctr;
                 B.img_base = reinterpret_cast<float *>(img_base);
                 B.img_step = (long long)step_img;
                 B.img_t0 = t0;
                 B.img_fmt = img_fmt;
+                const std::vector<uintptr_t> args = arg_words(amaps, B, mu, eta, P->d_tile_order);
                 if (int rc = capture_chunk(P, P->g_adj, key, args, C, step_ctr, -C, true, [&](int j, const GroupStreams &g) {
                         AdjArgs Bj = B;
                         Bj.it = j;

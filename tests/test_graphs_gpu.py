@@ -102,3 +102,62 @@ def test_batched_graphs_are_bit_identical(cuda_device):
     for o in (out, out2):
         for a, b in zip(o[0] + o[1], base[0] + base[1]):
             np.testing.assert_array_equal(a, b)
+
+
+def _plan_gradient(plan, t, res, ws, *, checkpoint_every, cached):
+    """dL/dvp through the C ABI on the caller's workspace ws; res: the
+    adjoint sources of p, vx, vz (None: unused)."""
+    import ctypes
+
+    from geobrain_b200 import _lib
+    from geobrain_b200.wave import engine
+    dev = t["vp"].device
+    n_ck = -(-(plan.geo.nt - cached) // checkpoint_every)
+    ck = torch.empty(max(n_ck * plan.checkpoint_bytes(plan.geo.nt, "fp32"), 256), dtype=torch.uint8, device=dev)
+    img = torch.empty(max(plan.imaging_bytes(cached, False, "fp32"), 256), dtype=torch.uint8, device=dev)
+    store = engine.make_store(ck if n_ck > 0 else None, checkpoint_every, "fp32", img, cached, False, "fp32")
+    engine.run_forward(plan, t["vp"], t["rho"], t["damp"], t["src_v"], want_energy=False, store=store)
+    g = torch.empty((plan.geo.nz, plan.geo.nx), device=dev)
+    _lib.check(plan._lib.gb_backward(plan.h, t["vp"].data_ptr(), t["rho"].data_ptr(), t["damp"].data_ptr(),
+                                     t["src_v"].data_ptr(), *[_lib.ptr(r) for r in res], ctypes.byref(store),
+                                     g.data_ptr(), None, None, ws.data_ptr(), ws.numel(), engine.stream_handle(dev)))
+    return g.cpu().numpy()
+
+
+@pytest.mark.parametrize("change", ["resident", "checkpoint_every"])
+def test_adjoint_graphs_follow_the_workspace_layout(cuda_device, change):
+    """Gradients of one plan by the tile adjoint in one caller-owned
+    workspace, before and after what moves the adjoint's buffers inside it:
+    another resident mode or tiling (vx residuals keep the adjoint in the
+    tile kernels), or another segment length of a partial cache.  Each equals
+    a plan that never ran anything else, bit for bit."""
+    from geobrain_b200.wave import engine
+    c = _unique_receivers(synthetic_case(60, 200, 10, 55, 2, seed=53))
+    t = {k: torch.as_tensor(c[k], device=cuda_device) for k in ("vp", "rho", "damp", "src_v")}
+    shape = (2, c["nt"], len(c["rcv_x"]))
+    rng = np.random.default_rng(9)
+    rp, rv = (torch.as_tensor(rng.standard_normal(shape).astype(np.float32), device=cuda_device) for _ in range(2))
+    geo = engine.Geometry(c["nz"], c["nx"], c["nabc"], c["nt"], c["dt"], c["dx"], 2, False)
+    new = lambda: engine.Plan(geo, c["src_x"], c["src_z"], c["rcv_x"], c["rcv_z"])
+    if change == "resident":
+        runs = [(("auto", 0), 55, 55), ((False, 0), 55, 55), (("cluster", 0), 55, 55), (("global", 16), 55, 55),
+                (("auto", 0), 55, 55)]
+    else:
+        runs = [((False, 0), k, 33) for k in (5, 11, 3, 5)]
+
+    def bytes_of(plan, run):
+        plan.set_resident(*run[0])
+        return plan.gradient_workspace_bytes(False, max(1, min(run[1], c["nt"] - run[2])), "fp32")
+
+    plan = new()
+    sizes = [bytes_of(plan, r) for r in runs]
+    assert len(set(sizes)) > 2                 # the layouts do differ
+    ws = torch.empty(max(sizes), dtype=torch.uint8, device=cuda_device)
+    for mode, every, cached in runs:
+        fresh = new()
+        for p in (plan, fresh):
+            p.set_resident(*mode)
+        base = _plan_gradient(fresh, t, (rp, rv, None), torch.empty_like(ws), checkpoint_every=every, cached=cached)
+        out = _plan_gradient(plan, t, (rp, rv, None), ws, checkpoint_every=every, cached=cached)
+        assert np.abs(base).max() > 0
+        np.testing.assert_array_equal(out, base, err_msg=f"{mode} {every}")
