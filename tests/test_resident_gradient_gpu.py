@@ -66,3 +66,36 @@ def test_resident_gradient_is_the_tile_kernels(cuda_device, shape, tile_rows, or
     for a, b in zip(out, base):
         assert np.abs(b).max() > 0
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("order,fmt,free_surface,rho", [(4, "fp32", False, False), (8, "fp24", True, True)])
+def test_resident_adjoint_reads_what_the_tile_forward_wrote(cuda_device, order, fmt, free_surface, rho):
+    """The adjoint's kernel is chosen when the backward runs: after
+    set_resident between the two, the resident adjoint reads a store the tile
+    forward made, which holds no imaging fields off the pressure mask.  With
+    the store's bytes all ones before the forward (NaN in every format) the
+    gradient is the one of a tile forward and a tile adjoint."""
+    from geobrain_b200.wave import engine
+    c = synthetic_case(70, 245, 9, 33, 1, seed=19, free_surface=free_surface)
+    _, keep = np.unique(c["rcv_z"] * 100003 + c["rcv_x"], return_index=True)
+    keep = np.sort(keep)[c["rcv_z"][np.sort(keep)] != -1]
+    c["src_x"], c["src_z"] = np.array([c["nx"] // 2]), np.array([3])
+    c["rcv_x"], c["rcv_z"] = c["rcv_x"][keep], c["rcv_z"][keep]
+    t = {k: torch.as_tensor(c[k], device=cuda_device) for k in ("vp", "rho", "damp", "src_v")}
+    geo = engine.Geometry(c["nz"], c["nx"], c["nabc"], c["nt"], c["dt"], c["dx"], order // 2, free_surface)
+    plan = engine.Plan(geo, c["src_x"], c["src_z"], c["rcv_x"], c["rcv_z"])
+    img = torch.full((plan.imaging_bytes(c["nt"], rho, fmt),), 255, dtype=torch.uint8, device=cuda_device)
+    store = engine.make_store(None, c["nt"], "fp32", img, c["nt"], rho, fmt)
+    plan.set_resident(False)
+    p, *_ = engine.run_forward(plan, t["vp"], t["rho"], t["damp"], t["src_v"], want_energy=False, store=store)
+    res = torch.randn(p.shape, generator=torch.Generator().manual_seed(5)).to(cuda_device)
+    args = (plan, t["vp"], t["rho"], t["damp"], t["src_v"], res, None, None, store, rho)
+    base = engine.run_backward(*args)
+    assert float(base[0].abs().max()) > 0
+    plan.set_resident("global", 16)
+    plan.set_profiling(True)
+    out = engine.run_backward(*args)
+    assert plan.profile()["launches"] < c["nt"]          # one launch for all steps
+    for a, b in zip(out, base):
+        if b is not None:
+            np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
