@@ -284,15 +284,16 @@ def full_cache_bytes(plan, with_rho: bool, imaging_dtype: str) -> int:
             plan.gradient_workspace_bytes(with_rho, 1, imaging_dtype) + 4 * S * nt * NR * 4)
 
 
-def batch_hold_bytes(plans, with_rho: bool, imaging_dtype: str) -> int:
-    """Device bytes a fused batched gradient of these models holds at once, at
-    its fullest: the imaging fields, the larger of the forward's and the
-    adjoint's workspaces (one is given back before the other is taken) and
-    two trace fields."""
+def batch_hold_blocks(plans, with_rho: bool, imaging_dtype: str):
+    """What a fused batched gradient of these models holds at its fullest: the
+    sizes of its large blocks (one with the imaging fields of every model; per
+    model the larger of the forward's and the adjoint's workspace, of which
+    one is given back before the other is taken), and the bytes of the traces:
+    per model three recorded fields and three of the residual and what it
+    takes to form it."""
     img = sum(_align256(p.imaging_bytes(p.geo.nt, with_rho, imaging_dtype)) for p in plans)
-    fwd = sum(p.workspace_bytes(False, 0) for p in plans)
-    adj = sum(p.gradient_workspace_bytes(with_rho, 1, imaging_dtype) for p in plans)
-    return img + max(fwd, adj) + sum(2 * p.n_shots * p.geo.nt * p.n_rcv * 4 for p in plans)
+    ws = [max(p.workspace_bytes(False, 0), p.gradient_workspace_bytes(with_rho, 1, imaging_dtype)) for p in plans]
+    return [img, *ws], sum(6 * p.n_shots * p.geo.nt * p.n_rcv * 4 for p in plans)
 
 
 def plan_sub_batches(sizes: Sequence[int], avail: int) -> List[List[int]]:
@@ -344,7 +345,9 @@ def acoustic_gradient_batched(models: Sequence[dict], residual, *, fd_order: int
     sub-batch starts.  Nothing is recomputed unless one model alone does not
     fit, in which case that model keeps checkpoints (in `snapshot_dtype`)
     for the steps that do not.  memory_budget: the bytes a sub-batch may
-    hold (default: the free device memory less 2 GiB and 5 %).  Under
+    hold.  By default the models are one sub-batch where the unused blocks of
+    torch's allocator hold it, as after an earlier call, else a sub-batch may
+    hold the free device memory, those blocks included, less 2 GiB and 5 %.  Under
     autograd (acoustic_forward_batched and loss.backward()) every model's
     store must survive until the backward, so
     an ensemble larger than the device memory recomputes its uncached steps;
@@ -367,14 +370,13 @@ def acoustic_gradient_batched(models: Sequence[dict], residual, *, fd_order: int
     vps = [_as_f32(m["vp"].detach() if torch.is_tensor(m["vp"]) else m["vp"], device, "vp") for m in models]
     rhos = [_as_f32(m["rho"].detach() if torch.is_tensor(m["rho"]) else m["rho"], device, "rho") for m in models]
     sizes = [full_cache_bytes(p, with_rho, imaging_dtype) for p in prep.plans]
-    pool = engine.unused_pool(device)
     if memory_budget is not None:
         avail = int(memory_budget)
-    elif batch_hold_bytes(prep.plans, with_rho, imaging_dtype) <= pool:
+    elif engine.pool_holds(device, *batch_hold_blocks(prep.plans, with_rho, imaging_dtype)):
         avail = sum(sizes)               # one sub-batch, out of what the allocator holds unused
     else:
         free, _ = torch.cuda.mem_get_info(device)
-        avail = free + pool
+        avail = free + engine.unused_pool(device)
         avail -= (2 << 30) + avail // 20
     losses = torch.zeros(n, dtype=torch.float32, device=device)
     grads_vp, grads_rho = [None] * n, [None] * n

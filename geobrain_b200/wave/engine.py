@@ -303,11 +303,30 @@ def choose_checkpoint_every(plan: Plan, checkpoint_segments: int = 1, checkpoint
 
 
 def unused_pool(device) -> int:
-    """Bytes torch's caching allocator holds on the device and does not use:
-    memory that is there for certain, known without asking the driver
-    (cudaMemGetInfo took between 0.1 and 70 ms a call on a shared host,
-    against 2 ms for the rest of a gradient's host work)."""
+    """Bytes torch's caching allocator holds on the device and does not use,
+    over all its blocks (of any size, stream or private pool)."""
     return torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+
+
+def pool_holds(device, blocks: Sequence[int], other: int = 0) -> bool:
+    """Whether the allocator's unused memory holds a call that needs `blocks`
+    (the sizes of its large allocations) and `other` bytes at its fullest,
+    with 1/128 of their sum to spare; then there is no need to ask the driver
+    (cudaMemGetInfo took between 0.1 and 70 ms a call on a shared host,
+    against 2 ms for the rest of a gradient's host work).  The sum alone
+    cannot tell: unused blocks may be too small, or another stream's.  So the
+    blocks are allocated, together, and given back (20 us).  The spare part is
+    for what else the program allocates meanwhile; a call like an earlier one
+    finds 1.5 % more than it needs or above (the earlier forward's workspace)."""
+    total = sum(blocks) + other
+    if total + total // 128 > unused_pool(device):
+        return False
+    try:
+        held = [workspace(b, device) for b in blocks]
+    except torch.OutOfMemoryError:
+        return False
+    del held
+    return True
 
 
 def choose_cached_steps(plan: Plan, imaging_cache, with_rho: bool, device, imaging_fmt: str = "fp32",
@@ -318,7 +337,9 @@ def choose_cached_steps(plan: Plan, imaging_cache, with_rho: bool, device, imagi
     remaining steps, the workspaces, the trace gradients and a margin (2 GiB
     + 5 %) fit in the device memory available right now, counting blocks the
     caching allocator holds unused (GEOBRAIN_B200_IMAGING_CACHE_BYTES
-    overrides it with a byte budget).  memory_budget caps that available
+    overrides it with a byte budget).  Unused blocks that hold every step's
+    fields and all else the gradient needs (pool_holds), as after an earlier
+    call, settle it without asking the driver.  memory_budget caps the available
     memory (bytes the whole gradient may hold beyond what is allocated now)."""
     nt = plan.geo.nt
     per = max(plan.imaging_bytes(1, with_rho, imaging_fmt), 1)
@@ -341,16 +362,16 @@ def choose_cached_steps(plan: Plan, imaging_cache, with_rho: bool, device, imagi
         return (c * per + -(-rest // K) * one_ck + plan.gradient_workspace_bytes(with_rho, seg, imaging_fmt) +
                 plan.workspace_bytes(0, 0) + traces)
 
-    # every step's fields, the larger of the two workspaces (the forward's is
-    # given back before the adjoint's is taken) and a trace field fit in what
-    # the allocator holds unused, as after an earlier call: no need to ask
-    pool = unused_pool(device)
-    if memory_budget is None and nt * per + max(plan.workspace_bytes(0, 0),
-                                                plan.gradient_workspace_bytes(with_rho, 1, imaging_fmt)) + traces // 3 <= pool:
+    # at its fullest: every step's fields, the larger of the two workspaces (the
+    # forward's is given back before the adjoint's is taken), three recorded
+    # trace fields and three of the loss's gradient and what it takes to form it
+    if memory_budget is None and pool_holds(
+            device, [nt * per, max(plan.workspace_bytes(0, 0), plan.gradient_workspace_bytes(with_rho, 1, imaging_fmt)),
+                     *[traces // 3] * 6]):
         return nt
     free, _ = torch.cuda.mem_get_info(device)
     # blocks torch's allocator holds but does not use are free for this too
-    avail = free + pool
+    avail = free + unused_pool(device)
     if memory_budget is not None:
         avail = min(avail, int(memory_budget))
     margin = (2 << 30) + avail // 20

@@ -83,14 +83,16 @@ class _Run3:
 def _imaging_fits(run, nbytes: int) -> bool:
     """Whether nbytes of imaging fields, the adjoint's workspace and a margin
     (2 GiB + 5 %) fit in the device memory available now (counting blocks the
-    caching allocator holds unused, which alone are enough after an earlier
-    call: the driver is asked only when they are not)."""
+    caching allocator holds unused; where those alone hold the gradient at its
+    fullest, four recorded trace fields and four of the loss's gradient
+    included, the driver is not asked)."""
     ws = int(run.L.gb3_backward_workspace_bytes(ctypes.byref(run.desc), 0, 1))
-    pool = engine.unused_pool(run.device)
-    if nbytes + ws + 4 * run.desc.n_shots * run.desc.nt * run.desc.n_rcv <= pool:
+    trace = 4 * run.desc.n_shots * run.desc.nt * run.desc.n_rcv
+    if engine.pool_holds(run.device, [nbytes, max(ws, int(run.L.gb3_workspace_bytes(ctypes.byref(run.desc)))),
+                                      *[trace] * 8]):
         return True
     free, _ = torch.cuda.mem_get_info(run.device)
-    avail = free + pool
+    avail = free + engine.unused_pool(run.device)
     return nbytes + ws + (2 << 30) + avail // 20 <= avail
 
 
