@@ -127,7 +127,7 @@ struct gb_plan {
     // 32-shot forward step, the adjoint unchanged).
     int sched = 0;
     std::vector<int4> sched_items;                 // forward work lists, one per launch configuration
-    std::vector<int> sched_off, sched_cnt;         // configuration g < n_groups: group g alone; n_groups: all
+    std::vector<int> sched_off, sched_cnt;         // configuration g < n_groups: group g's lane; n_groups: all groups
     std::vector<int> tile_order;                   // the tiles, slow path first
     std::vector<long long> sched_key;              // what the lists were built for
     int4 *d_items = nullptr;                       // this call's workspace copies (null: blockIdx order)
@@ -485,7 +485,7 @@ struct Layout {
 size_t img_esize(int f);
 
 // Room for the CTA schedule: the forward's work lists (each item split at
-// most once, for every group alone and for all groups together) and the
+// most once, for every lane of groups and for all groups together) and the
 // tile order.
 size_t sched_bytes(const gb_plan *p)
 {
@@ -664,15 +664,29 @@ cudaError_t launch_pdl(gb_plan *P, const void *fn, dim3 grid, size_t smem, void 
     return launch_kernel(P, fn, grid, dim3(NTHR), smem, args, st, true);
 }
 
-// The CTA schedule of a launch of groups [grp0, grp0 + grp_count): the
-// forward takes its work list (and its length as the grid), the adjoint the
-// tile order; launches of any other set of groups keep blockIdx order.
+// Lanes the shot groups of a plan run in: neighbouring groups share one, a
+// launch a step each.
+constexpr int kGroupLanes = 4;
+int group_lanes(const gb_plan *P)
+{
+    return P->group_streams ? std::max(1, std::min(P->n_groups, kGroupLanes)) : 1;
+}
+
+// lane i's groups: an even share of them
+inline void lane_groups(int i, int lanes, int n_groups, int *g0, int *gc)
+{
+    *g0 = (int)((long long)n_groups * i / lanes);
+    *gc = (int)((long long)n_groups * (i + 1) / lanes) - *g0;
+}
+
+// The CTA schedule of a launch of groups [grp0, grp0 + grp_count), a lane's or
+// all: the forward takes its work list (and its length as the grid), the
+// adjoint the tile order.
 void apply_schedule(const gb_plan *P, FwdArgs &A, int grp0, int grp_count, unsigned *grid)
 {
     A.items = nullptr;
     if (!P->d_items) return;
-    const int c = grp_count == 1 ? grp0 : (grp0 == 0 && grp_count == P->n_groups) ? P->n_groups : -1;
-    if (c < 0 || c >= (int)P->sched_cnt.size()) return;
+    const int c = grp_count == P->n_groups ? P->n_groups : grp0;
     A.items = P->d_items + P->sched_off[c];
     *grid = (unsigned)P->sched_cnt[c];
 }
@@ -723,14 +737,6 @@ struct GroupStreams {
     cudaStream_t at(int grp) const { return n == 1 ? main : P->gstream[grp]; }
 };
 
-// Lanes the shot groups of a plan run in: neighbouring groups share one, a
-// launch a step each.
-constexpr int kGroupLanes = 4;
-int group_lanes(const gb_plan *P)
-{
-    return P->group_streams ? std::max(1, std::min(P->n_groups, kGroupLanes)) : 1;
-}
-
 // want < 0: the lanes of the plan's groups; else `want` streams (the lanes of a batch)
 int group_streams(gb_plan *P, cudaStream_t main, GroupStreams *gs, int want = -1)
 {
@@ -774,11 +780,10 @@ int join(const GroupStreams &gs)
     return GB_OK;
 }
 
-// groups handled by one launch on stream i: an even share of them
+// groups handled by one launch on stream i
 inline void launch_groups(const GroupStreams &gs, int i, int n_groups, int *g0, int *gc)
 {
-    *g0 = (int)((long long)n_groups * i / gs.n);
-    *gc = (int)((long long)n_groups * (i + 1) / gs.n) - *g0;
+    lane_groups(i, gs.n, n_groups, g0, gc);
 }
 
 // the shots of groups [g0, g0 + gc)
@@ -993,18 +998,20 @@ void build_schedule(gb_plan *P, int slots)
     P->sched_items.clear();
     P->sched_off.clear();
     P->sched_cnt.clear();
-    const int concurrent = (P->group_streams && P->n_groups > 1) ? P->n_groups : 1;
-    for (int c = 0; c <= P->n_groups; ++c) {
-        const int g0 = c < P->n_groups ? c : 0, gc = c < P->n_groups ? 1 : P->n_groups;
-        const int per_launch = c < P->n_groups ? std::max(1, slots / concurrent) : slots;
+    // a list for each lane, which the configurations of its groups share, and one of all groups
+    const int lanes = std::min(P->n_groups, kGroupLanes), concurrent = group_lanes(P);
+    for (int i = 0; i <= lanes; ++i) {
+        int g0 = 0, gc = P->n_groups;
+        if (i < lanes) lane_groups(i, lanes, P->n_groups, &g0, &gc);
+        const int per_launch = i < lanes ? std::max(1, slots / concurrent) : slots;
         std::vector<int4> it;
         for (int t : P->tile_order)
             for (int g = g0; g < g0 + gc; ++g) it.push_back(make_int4(t, P->group_first(g), P->group_shots(g), 0));
-        P->sched_off.push_back((int)P->sched_items.size());
+        const int off = (int)P->sched_items.size();
         const int n = (int)it.size(), first_split = std::max(0, n - per_launch);
-        for (int i = 0; i < n; ++i) {
-            const int4 w = it[i];
-            if (i >= first_split && w.z >= 2) {
+        for (int k = 0; k < n; ++k) {
+            const int4 w = it[k];
+            if (k >= first_split && w.z >= 2) {
                 const int h = w.z / 2;
                 P->sched_items.push_back(make_int4(w.x, w.y, h, 0));
                 P->sched_items.push_back(make_int4(w.x, w.y + h, w.z - h, 0));
@@ -1012,7 +1019,8 @@ void build_schedule(gb_plan *P, int slots)
                 P->sched_items.push_back(w);
             }
         }
-        P->sched_cnt.push_back((int)P->sched_items.size() - P->sched_off.back());
+        P->sched_off.insert(P->sched_off.end(), i < lanes ? gc : 1, off);
+        P->sched_cnt.insert(P->sched_cnt.end(), i < lanes ? gc : 1, (int)P->sched_items.size() - off);
     }
 }
 

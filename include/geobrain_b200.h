@@ -132,8 +132,9 @@ int gb_plan_set_graph_steps(gb_plan *plan, int steps);
 int gb_plan_set_schedule(gb_plan *plan, int mode);
 
 /* The forward work list that schedule mode 1 builds for `slots` resident
- * CTAs (no device call).  config g < n_groups: the launch of shot group g
- * alone (group streams); config n_groups: one launch of every group.
+ * CTAs (no device call).  config g < n_groups: the launch that shot group g
+ * is in with group streams (alone up to four groups; more share the four
+ * streams, neighbours in a launch); config n_groups: one launch of every group.
  * Writes *n_items, and, when items is not NULL (cap >= *n_items), the items
  * as (tile, first shot, shots) triples. */
 int gb_plan_schedule_items(gb_plan *plan, int slots, int config, int32_t *items, int cap, int *n_items);

@@ -110,3 +110,29 @@ def test_schedule_items_refuses_bad_arguments(lib):
         assert lib.gb_plan_set_schedule(h, 2) == _lib.GB_E_ARG
     finally:
         lib.gb_plan_destroy(h)
+
+
+@pytest.mark.parametrize("shots,spc,slots", [(5, 1, 7), (7, 1, 37), (23, 2, 296)])
+def test_more_groups_than_streams_share_work_lists(lib, shots, spc, slots):  # noqa: F811
+    """Five groups or more run on four streams, an even share of neighbours
+    each: a group's work list is its stream's, every (tile, shot) is in the
+    list of one stream, and a quarter of the slots' last items are split."""
+    h = _plan(lib, 60, 250, 10, 4, shots)
+    try:
+        assert lib.gb_plan_set_tiling(h, 16, spc) == 0, lib.gb_last_error()
+        n_groups = -(-shots // spc)
+        n_tiles = -(-(250 + 20) // TX) * -(-(60 + 20) // 16)
+        edges = [n_groups * i // 4 for i in range(5)]
+        seen = []
+        for g0, g1 in zip(edges, edges[1:]):
+            it = _items(lib, h, slots, g0)
+            for g in range(g0 + 1, g1):
+                np.testing.assert_array_equal(_items(lib, h, slots, g), it)
+            assert {int(s) // spc for s in it[:, 1]} == set(range(g0, g1))
+            seen += [(int(t), s) for t, s0, ns in it for s in range(s0, s0 + ns)]
+            whole = (g1 - g0) * n_tiles                    # (tile, group) items before the split
+            last = [min(spc, shots - g * spc) for g in range(g0, g1)] * n_tiles
+            assert len(it) == whole + sum(n >= 2 for n in last[max(0, whole - max(1, slots // 4)):])
+        assert sorted(seen) == [(t, s) for t in range(n_tiles) for s in range(shots)]
+    finally:
+        lib.gb_plan_destroy(h)
