@@ -1801,13 +1801,15 @@ int gb_plan_autotune(gb_plan *P, const float *vp, const float *rho, const float 
                     }
             }
         }
+    // (a resident forward launches no step graphs: the plan's chunk length
+    // stays, for its gradients)
     if (!P->cpml)
         for (int tz : kResidentRows)
             if (P->res_fits(tz, gb_plan::sm_count())) {
-                cands.push_back({saved.tz, saved.spc, true, 0, false, tz, 1});
-                if (P->res_single_ok()) cands.push_back({saved.tz, saved.spc, true, 0, false, tz, 3});
+                cands.push_back({saved.tz, saved.spc, true, saved.graph, false, tz, 1});
+                if (P->res_single_ok()) cands.push_back({saved.tz, saved.spc, true, saved.graph, false, tz, 3});
                 const long long n = (long long)((P->Nx + TX - 1) / TX) * ((P->Nz + tz - 1) / tz);
-                if (n <= gb_plan::kMaxClusterTiles) cands.push_back({saved.tz, saved.spc, true, 0, false, tz, 2});
+                if (n <= gb_plan::kMaxClusterTiles) cands.push_back({saved.tz, saved.spc, true, saved.graph, false, tz, 2});
             }
     cudaEvent_t e0, e1;
     GB_CUDA(cudaEventCreate(&e0));

@@ -145,7 +145,9 @@ int gb_plan_schedule_items(gb_plan *plan, int slots, int config, int32_t *items,
  *   - shots per CTA automatic, 1, 2, 4, 8 or 16;
  *   - per-group streams on / off;
  *   - graph chunks of 16 steps or none;
- *   - the streaming forward kernel or the tile kernel.
+ *   - the streaming forward kernel or the tile kernel;
+ *   - the resident forwards that fit (their launches use no graph, and the
+ *     plan's chunk length stays as it is for its gradients).
  * It keeps the fastest on the plan and reports its time per step.  Each
  * candidate runs three times; the first is a warm-up.  The workspace must
  * hold gb_plan_autotune_workspace_bytes(plan); candidates that do not fit

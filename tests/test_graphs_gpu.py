@@ -161,3 +161,29 @@ def test_adjoint_graphs_follow_the_workspace_layout(cuda_device, change):
         out = _plan_gradient(plan, t, (rp, rv, None), ws, checkpoint_every=every, cached=cached)
         assert np.abs(base).max() > 0
         np.testing.assert_array_equal(out, base, err_msg=f"{mode} {every}")
+
+
+def test_gradient_after_autotuning_keeps_its_step_graphs(cuda_device):
+    """One shot on a small grid tunes to a resident forward, which uses no
+    step graphs; the plan's gradients keep theirs (or run resident too): few
+    host launch calls, and the untuned plan's numbers."""
+    c = _unique_receivers(synthetic_case(70, 200, 10, 96, 1, seed=57))
+    plan = _plan_of(c, 4)
+    base = _grad(c, cuda_device, imaging_cache="all")
+    try:
+        _grad(c, cuda_device, imaging_cache="all", autotune=True)
+        assert plan.config()["resident_rows"] > 0 and plan.config()["graph_steps"] == 16
+        plan.set_profiling(True)
+        out = _grad(c, cuda_device, imaging_cache="all")
+        assert plan.profile()["launch_calls"] < c["nt"] // 2
+    finally:
+        plan.set_profiling(False)
+        plan.tuned = None
+        plan.set_tiling(16, 0)
+        plan.set_graph_steps(16)
+        plan.set_group_streams(True)
+        plan.set_streaming(False)
+        plan.set_resident("auto")
+    for a, b in zip(out, base):
+        if b is not None:
+            np.testing.assert_array_equal(a, b)
