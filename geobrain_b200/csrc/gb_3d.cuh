@@ -517,35 +517,47 @@ __global__ void __launch_bounds__(128, RHO ? 4 : 5) adj_v3_kernel(const AdjArgs3
 // p[fs-1] = -p[fs+1]: minus the receivers in that one and minus its share of
 // the divergence, c2 mu_vz[fs] (all else there is zero).  A source in the
 // mirror plane is overwritten by the mirror: zero.
-__global__ void wavelet_grad3_kernel(const AdjArgs3 A, const int *src, const int *rcv, const float *res_p,
-                                     float *grad_wavelet, float *off, int it)
+// One block per shot: a source off the mask looks through all receivers at
+// every step.  (Gradient of one shot, 56 x 80 x 80 cells, 20 steps, 4096
+// receivers: 5.95 ms with one thread a shot, 1.71 with a block, 1.65 for a
+// source on the mask.)
+constexpr int kWaveletThreads = 256;
+__global__ void __launch_bounds__(kWaveletThreads)
+wavelet_grad3_kernel(const AdjArgs3 A, const int *src, const int *rcv, const float *res_p, float *grad_wavelet,
+                     float *off, int it)
 {
     const Geo3 &g = A.g;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= g.n_shots) return;
+    const int s = blockIdx.x;
     const int z = src[s], y = src[g.n_shots + s], x = src[2 * g.n_shots + s];
     const long long o = (long long)z * g.plane + (long long)y * g.pitch + x;
     const float *P = A.mu + (long long)s * 4 * g.vol;
-    float lam;
-    if (in_p(g, z, y, x)) {
-        lam = P[o] / A.a1[o];
-    } else if (A.free_surface && z == g.fs - 1) {
+    const bool on_mask = in_p(g, z, y, x), overwritten = A.free_surface && z == g.fs - 1;
+    const bool mirrored = A.free_surface && z == g.fs + 1;
+    float lam = 0.f;
+    if (!on_mask && !overwritten && res_p) {
+        __shared__ float part[kWaveletThreads / 32];
+        for (int r = threadIdx.x; r < g.n_rcv; r += kWaveletThreads)
+            if (rcv[g.n_rcv + r] == y && rcv[2 * g.n_rcv + r] == x) {
+                const float v = res_p[((long long)s * g.nt + it) * g.n_rcv + r];
+                if (rcv[r] == z) lam += v;
+                if (mirrored && rcv[r] == g.fs - 1) lam -= v;
+            }
+        for (int d = 16; d > 0; d >>= 1) lam += __shfl_down_sync(0xffffffffu, lam, d);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = lam;
+        __syncthreads();
         lam = 0.f;
-    } else {
+        for (int i = 0; i < kWaveletThreads / 32; ++i) lam += part[i];
+    }
+    if (threadIdx.x != 0) return;
+    if (on_mask) {
+        lam = P[o] / A.a1[o];
+    } else if (!overwritten) {
         auto at = [&](int f, int zz, int yy, int xx) {
             return zz < 0 || zz >= g.Nz || yy < 0 || yy >= g.Ny || xx < 0 || xx >= g.Nx
                        ? 0.f
                        : P[(long long)f * g.vol + (long long)zz * g.plane + (long long)yy * g.pitch + xx];
         };
-        const bool mirrored = A.free_surface && z == g.fs + 1;
-        lam = off[s];
-        if (res_p)
-            for (int r = 0; r < g.n_rcv; ++r)
-                if (rcv[g.n_rcv + r] == y && rcv[2 * g.n_rcv + r] == x) {
-                    const float v = res_p[((long long)s * g.nt + it) * g.n_rcv + r];
-                    if (rcv[r] == z) lam += v;
-                    if (mirrored && rcv[r] == g.fs - 1) lam -= v;
-                }
+        lam += off[s];
         lam += d4f(at(1, z, y, x), at(1, z, y, x - 1), at(1, z, y, x + 1), at(1, z, y, x - 2)) +
                d4f(at(2, z, y, x), at(2, z, y - 1, x), at(2, z, y + 1, x), at(2, z, y - 2, x)) +
                d4f(at(3, z, y, x), at(3, z - 1, y, x), at(3, z + 1, y, x), at(3, z - 2, y, x));

@@ -523,8 +523,8 @@ int gb3_backward(const gb3_model_desc *desc, const int64_t *src_x, const int64_t
             adj_p3_kernel<<<grid, block, 0, st>>>(A);
             if (g.n_rcv > 0 && res_p) inj3_kernel<<<nb, 256, 0, st>>>(A, d_rcv, res_p, res_vx, res_vy, res_vz, 1, it);
             if (grad_wavelet)
-                wavelet_grad3_kernel<<<(g.n_shots + 127) / 128, 128, 0, st>>>(A, d_src, d_rcv, g.n_rcv > 0 ? res_p : nullptr,
-                                                                              grad_wavelet, off, it);
+                wavelet_grad3_kernel<<<g.n_shots, kWaveletThreads, 0, st>>>(A, d_src, d_rcv, g.n_rcv > 0 ? res_p : nullptr,
+                                                                            grad_wavelet, off, it);
             if (with_rho) adj_v3_kernel<true><<<grid, block, 0, st>>>(A);
             else adj_v3_kernel<false><<<grid, block, 0, st>>>(A);
             GB_CUDA(cudaGetLastError());

@@ -407,3 +407,32 @@ def test_cuda_3d_wavelet_gradient_of_border_sources_below_the_surface(cuda_devic
     assert orc.rel_l2(v.grad.cpu().numpy(), gv) < 1e-4
     for i in range(4):
         assert orc.rel_l2(s.grad[i].cpu().numpy(), gw[i]) < 1e-4, i
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_rcv", [1, 255, 257, 700])
+def test_cuda_3d_wavelet_gradient_searches_all_receivers(cuda_device, n_rcv):
+    """A source off the pressure mask with receivers in its cell among many
+    (the first, the last and some between): the kernel's threads share the
+    search.  Against the float64 oracle, 1e-4 as above."""
+    from geobrain_b200.wave import acoustic_forward_kernel_3d, bc_pml_3d
+    rng = np.random.default_rng(29)
+    nz, ny, nx, nabc, nt = 9, 8, 11, 4, 24
+    vp = (2000 + 800 * rng.random((nz, ny, nx))).astype(np.float32)
+    rho = np.full((nz, ny, nx), 2100.0, np.float32)
+    damp = bc_pml_3d(nx, ny, nz, 10.0, 10.0, 10.0, nabc, float(vp.max()), free_surface=False).astype(np.float32)
+    w = rng.standard_normal((2, nt)).astype(np.float32)
+    src = dict(src_x=np.array([1 - nabc, 5]), src_y=np.array([3, 4]), src_z=np.array([2, 2]), src_v=w)
+    rcv = dict(rcv_x=rng.integers(0, nx, n_rcv), rcv_y=rng.integers(0, ny, n_rcv), rcv_z=rng.integers(0, nz, n_rcv))
+    for i in {0, n_rcv // 3, n_rcv // 2, n_rcv - 1}:
+        rcv["rcv_x"][i], rcv["rcv_y"][i], rcv["rcv_z"][i] = 1 - nabc, 3, 2
+    kw = dict(nz=nz, ny=ny, nx=nx, nt=nt, dt=1e-3, nabc=nabc, free_surface=False, **rcv)
+    res = rng.standard_normal((2, nt, n_rcv)).astype(np.float32)
+    t = lambda a: torch.as_tensor(a, device=cuda_device)
+    s = t(w).requires_grad_(True)
+    out = acoustic_forward_kernel_3d(dx=10.0, dy=10.0, dz=10.0, src_n=2, rcv_n=n_rcv, damp=t(damp), vp=t(vp),
+                                     rho=t(rho), device=cuda_device, **kw, **dict(src, src_v=s))
+    (t(res) * out["p"]).sum().backward()
+    _, _, gw = o3.gradient(dz=10.0, damp=damp, vp=vp, rho=rho, with_wavelet=True, res_p=res, **kw, **src)
+    for i in range(2):
+        assert orc.rel_l2(s.grad[i].cpu().numpy(), gw[i]) < 1e-4, i
