@@ -476,7 +476,7 @@ namespace {
 // Workspace layout (offsets in bytes from the 256-aligned base).
 struct Layout {
     size_t err, coef, fields, energy, src, rcv_ptr, rcv_ent, tile_fast, sched, amax, cpml, psi, total;
-    size_t res_ptr, res_ent, res_x;           // resident forward: receiver CSR, exchange strips
+    size_t res_ptr, res_ent, res_x;           // resident kernels: receiver CSR, exchange strips
     // gradient only
     size_t mu, eta, img, g1, c1, g2, c2, arcv_ptr, arcv_ent;
     int n_img;
@@ -502,7 +502,8 @@ Layout layout(const gb_plan *p, int with_gradient = 0, int checkpoint_every = 0,
     const size_t S = p->d.n_shots;
     L.err = o; o += 256;
     L.coef = o; o = align256(o + 5 * p->plane * 4);
-    L.fields = o; o = align256(o + 2 * S * 3 * p->plane * 4);
+    const size_t state = 2 * S * 3 * p->plane * 4;
+    if (with_gradient == 0) L.fields = o, o = align256(o + state);
     L.energy = o; o = align256(o + 3 * p->plane * 4);
     L.src = o; o = align256(o + 2 * S * 4);
     L.rcv_ptr = o; o = align256(o + (p->n_tiles + 1) * 4);
@@ -514,19 +515,26 @@ Layout layout(const gb_plan *p, int with_gradient = 0, int checkpoint_every = 0,
         L.cpml = o; o = align256(o + (4 * (size_t)p->Nz + 4 * (size_t)p->pitch) * 4);
         L.psi = o; o = align256(o + 2 * S * 4 * p->plane * 4);   // two levels of the memory variables
     }
+    // the resident kernels' regions; a gradient's adjoint runs either those or
+    // the tile kernels, so there they share the place of what only the latter
+    // use: the recomputed state, the adjoint state and the segment buffer
+    size_t res_end = 0;
     if (p->res_tz > 0) {
         const ResidentKernel k = resident_kernel(p->R, p->res_tz, p->res_single ? 2 : 0);
-        L.res_ptr = o; o = align256(o + (p->res_n + 1) * 4);
-        L.res_ent = o; o = align256(o + std::max<size_t>(p->d.n_rcv, 1) * 16);
-        L.res_x = o; o = align256(o + S * p->res_n * k.tile_words * 8);
+        L.res_ptr = o;
+        L.res_ent = align256(L.res_ptr + (p->res_n + 1) * 4);
+        L.res_x = align256(L.res_ent + std::max<size_t>(p->d.n_rcv, 1) * 16);
+        res_end = align256(L.res_x + S * p->res_n * k.tile_words * 8);
+        if (with_gradient == 0) o = res_end;
     }
     L.n_img = with_gradient >= 2 ? 3 : 1;
     if (with_gradient > 0) {
         const size_t K = std::max(1, std::min(checkpoint_every, p->d.nt));
         const size_t G = p->n_groups;
-        L.mu = o; o = align256(o + S * 2 * 3 * p->plane * 4);
+        L.fields = o; o = align256(o + state);
+        L.mu = o; o = align256(o + state);
         if (p->cpml) L.eta = o, o = align256(o + S * 2 * 4 * p->plane * 4);   // adjoints of the memory variables
-        L.img = o; o = align256(o + K * L.n_img * S * p->plane * img_esize(img_fmt));
+        L.img = o; o = std::max(res_end, align256(o + K * L.n_img * S * p->plane * img_esize(img_fmt)));
         L.g1 = o; o = align256(o + G * p->plane * 4);
         L.c1 = o; o = align256(o + G * p->plane * 4);
         if (with_gradient >= 2) {

@@ -68,3 +68,22 @@ def test_modes_and_refusals(lib):
     finally:
         for p in (h, h8, hfs):
             lib.gb_plan_destroy(p)
+
+
+@pytest.mark.parametrize("nz,nx,nabc,half,shots", [
+    (100, 200, 20, 2, 1), (100, 200, 20, 4, 8), (400, 1200, 30, 4, 1), (60, 300, 12, 2, 4), (88, 200, 20, 4, 5)])
+@pytest.mark.parametrize("with_rho", [0, 1])
+def test_gradients_need_no_memory_for_the_resident_kernels(lib, nz, nx, nabc, half, shots, with_rho):  # noqa: F811
+    """A gradient's adjoint runs the resident kernel or the tile kernels, in
+    one place of the workspace: a plan with a resident tiling asks for no more
+    than one without, and so keeps as many steps within a memory budget."""
+    h = _plan(lib, nz, nx, nabc, half, shots)
+    try:
+        assert _resident(lib, h)[0] > 0
+        sizes = []
+        for mode in (-1, 0):
+            assert lib.gb_plan_set_resident(h, mode, 0) == 0
+            sizes.append(lib.gb_plan_gradient_workspace_bytes(h, with_rho, 1, 0))
+        assert sizes[0] == sizes[1] > 0
+    finally:
+        lib.gb_plan_destroy(h)
