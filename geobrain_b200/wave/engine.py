@@ -311,15 +311,16 @@ def unused_pool(device) -> int:
 def pool_holds(device, blocks: Sequence[int], other: int = 0) -> bool:
     """Whether the allocator's unused memory holds a call that needs `blocks`
     (the sizes of its large allocations) and `other` bytes at its fullest,
-    with 1/128 of their sum to spare; then there is no need to ask the driver
+    with 1/256 of their sum to spare; then there is no need to ask the driver
     (cudaMemGetInfo took between 0.1 and 70 ms a call on a shared host,
     against 2 ms for the rest of a gradient's host work).  The sum alone
     cannot tell: unused blocks may be too small, or another stream's.  So the
     blocks are allocated, together, and given back (20 us).  The spare part is
     for what else the program allocates meanwhile; a call like an earlier one
-    finds 1.5 % more than it needs or above (the earlier forward's workspace)."""
+    finds 0.6 % more than it needs or above (blocks are rounded up, and the
+    earlier forward's workspace is there too)."""
     total = sum(blocks) + other
-    if total + total // 128 > unused_pool(device):
+    if total + total // 256 > unused_pool(device):
         return False
     try:
         held = [workspace(b, device) for b in blocks]

@@ -55,7 +55,7 @@ def test_unused_blocks_must_hold_every_trace_field(monkeypatch, fields):
 def test_unused_blocks_that_hold_a_gradient_settle_it(monkeypatch):
     plan = _plan()
     fixed, trace = _needs(plan)
-    mem = _Memory(monkeypatch, (fixed + 6 * trace) * 129 // 128 + 1)
+    mem = _Memory(monkeypatch, (fixed + 6 * trace) * 257 // 256 + 1)
     assert _choose(plan) == plan.geo.nt and mem.asked == 0
 
 
@@ -84,5 +84,5 @@ def test_batched_and_3d_gradients_count_their_traces(monkeypatch):
     need = 100000 + 3000 + 8 * 4 * 2 * 50 * 30
     mem = _Memory(monkeypatch, need)
     assert not kernel3d._imaging_fits(Run, 100000) and mem.asked == 1
-    mem = _Memory(monkeypatch, need * 129 // 128 + 1)
+    mem = _Memory(monkeypatch, need * 257 // 256 + 1)
     assert kernel3d._imaging_fits(Run, 100000) and mem.asked == 0
