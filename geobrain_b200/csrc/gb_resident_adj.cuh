@@ -164,9 +164,7 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_adj_kernel(const ResArgs 
     C.fast = res_load_coef<R, NW, TZ>(A, cf, z0, x0);
 
     // this thread's 4-cell groups: c < LI interior row ri + c of its lane,
-    // c = LI its boundary item; element offset of each in a plane (-1: none),
-    // and in bit c of on_p whether any of its cells is on the p mask (the tile
-    // forward, which may have made the store, writes I for those only)
+    // c = LI its boundary item; element offset of each in a plane (-1: none)
     const bool ilane = lane >= 2 && lane <= 29;
     const int ri = 2 * R + warp * G::LI;
     const bool interior = G::NI > 0 && ilane && ri < TZ;
@@ -176,21 +174,19 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_adj_kernel(const ResArgs 
     ResRecv<R, NW, TZ> recv;
     recv.init(sP, sVX, sVZ, xb, K.nb);
     int off[NC];
-    unsigned on_p = 0;
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         const int r = c < G::LI ? ri + c : br, l = c < G::LI ? lane : bl;
         const bool mine = c < G::LI ? interior && ri + c < TZ : item;
         const int gz = z0 - R + r, gx = x0 - 4 + 4 * l;
         off[c] = mine && gz < g.Nz && gx < g.Nx ? gz * g.pitch + gx : -1;
-        if (off[c] >= 0 && gz >= g.p_r0 && gz <= g.p_r1 && gx + 3 >= g.p_c0 && gx <= g.p_c1) on_p |= 1u << c;
     }
     const long long so = (long long)s * g.plane;
     ImgRaw im[NC], jx[RHO ? NC : 1], jz[RHO ? NC : 1];
     const auto load_i = [&](int it) {
 #pragma unroll
         for (int c = 0; c < NC; ++c)
-            im[c] = (on_p >> c) & 1u ? load_img_raw(res_img_step(A, it), so + off[c], A.img_fmt) : img_raw_zero();
+            im[c] = off[c] >= 0 ? load_img_raw(res_img_step(A, it), so + off[c], A.img_fmt) : img_raw_zero();
     };
     const auto load_j = [&](int it) {
 #pragma unroll
@@ -306,11 +302,17 @@ __global__ void __launch_bounds__(NW * 32, 1) resident_adj_kernel(const ResArgs 
         // the next step writes mu_p, which this one's stencils read
         __syncthreads();
     }
+    // G1 and C1 hold zeros: groups wholly off the p mask stay so.  Their sums
+    // are zeros times whatever is in a store that the tile forward made, which
+    // writes I on the mask only.
 #pragma unroll
     for (int c = 0; c < NC; ++c)
         if (off[c] >= 0) {
-            stg4(A.G1 + so + off[c], s1[c]);
-            stg4(A.C1 + so + off[c], c1[c]);
+            const int gz = z0 - R + (c < G::LI ? ri + c : br), gx = x0 - 4 + 4 * (c < G::LI ? lane : bl);
+            if (gz >= g.p_r0 && gz <= g.p_r1 && gx + 3 >= g.p_c0 && gx <= g.p_c1) {
+                stg4(A.G1 + so + off[c], s1[c]);
+                stg4(A.C1 + so + off[c], c1[c]);
+            }
             if (RHO) {
                 stg4(A.G2 + so + off[c], s2[c]);
                 stg4(A.C2 + so + off[c], c2[c]);
