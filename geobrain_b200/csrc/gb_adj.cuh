@@ -187,7 +187,9 @@ __device__ __forceinline__ void adj_body(const CUtensorMap *mP, const CUtensorMa
     const int vb = warp * G::LV, vcnt = TZ == NWARP * G::LV ? G::LV : min(G::LV, TZ - vb);
     const bool vlane = lane >= 1 && lane <= 30;
 
-    // per-thread partial sums over this CTA's shots (tile cells)
+    // per-thread partial sums over this CTA's shots (tile cells), in plain fp32:
+    // the gradient's error against float64 is the same with 1 to 16 shots
+    // (48 gradients of 200 steps: log ratios within 0.002 +- 0.001)
     float4 acc1[G::LV], acc2[G::LV];
 #pragma unroll
     for (int u = 0; u < G::LV; ++u) {

@@ -427,6 +427,10 @@ struct gb_plan {
     // from 592 on), and one group has no other beside it while its launches
     // end and start: a tenth slower, two groups 3 %.  With CPML the ends are
     // layer tiles, which take about twice an interior one's time: 1.2 more.
+    // (592 and 296 are four and two CTAs on each of a B200's 148 SMs, the fill
+    // is a fit to 16-row tiles.  With 32-row tiles, one CTA an SM, the choice
+    // measured 1.00 to 1.11 times the rate of the fewest groups of up to 8
+    // shots that make 592 CTAs, over 9 grids, forward and gradient.)
     // Gradient, ms, each against the choice before it:
     //   128 x 240, 40 shots, 300 steps: 2 a CTA 7.33, 1 a CTA 7.87
     //   240 x 540, 12 shots, 200 steps: 2 a CTA 5.60, 1 a CTA 6.68
