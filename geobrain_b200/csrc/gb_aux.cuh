@@ -119,8 +119,8 @@ __global__ void unpack16_kernel(const H *__restrict__ in, const float *__restric
 }
 
 // Checkpoint snapshots in 24 bits: the upper 24 bits of each fp32 (sign,
-// exponent, 15-bit mantissa) rounded to nearest even, 4 values to 3 words,
-// the same packing as the fp24 imaging fields.  The exponent is kept, so no
+// exponent, 15-bit mantissa) rounded to nearest even, packed as the fp24
+// imaging fields (store_img4).  The exponent is kept, so no
 // scale is needed; the relative error of each value is at most 2^-16.
 __global__ void pack24_kernel(const float *__restrict__ x, long long n4, float *__restrict__ out)
 {

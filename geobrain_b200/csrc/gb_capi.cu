@@ -1122,6 +1122,13 @@ int check_store(const gb_plan *P, const gb_grad_store *store)
     if (store->cached_steps > 0 && !store->imaging) return fail(GB_E_ARG, "cached_steps > 0 needs an imaging buffer");
     if (!img_format_ok(store->imaging_format))
         return fail(GB_E_ARG, "imaging_format must be GB_IMG_F32, GB_IMG_BF16 or GB_IMG_F24");
+    // the kernels' accesses: float4, or the uint2 of a quad's 16-bit values or upper halves
+    if (store->cached_steps > 0 &&
+        reinterpret_cast<uintptr_t>(store->imaging) % (store->imaging_format == GB_IMG_F32 ? 16 : 8))
+        return fail(GB_E_ARG, "the imaging buffer must start on a 16-byte boundary (8-byte for bf16 and f24)");
+    if (store->cached_steps < P->d.nt && store->format == GB_CKPT_F24 &&
+        reinterpret_cast<uintptr_t>(store->checkpoints) % 8)
+        return fail(GB_E_ARG, "f24 checkpoints must start on an 8-byte boundary");
     if (store->cached_steps < P->d.nt && !store->checkpoints) return fail(GB_E_ARG, "checkpoint storage missing");
     return GB_OK;
 }

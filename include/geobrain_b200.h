@@ -66,11 +66,13 @@ typedef struct gb_model_desc {
  * torch.utils.checkpoint segments of acoustic_2d.py:430,448-460):
  *   checkpoints       full state every checkpoint_every steps, in `format`,
  *                     gb_plan_checkpoint_bytes(plan, checkpoint_every, format)
- *                     bytes (may be NULL when cached_steps == nt);
+ *                     bytes (may be NULL when cached_steps == nt), f24 ones on
+ *                     an 8-byte boundary;
  *   imaging           the imaging fields of the last cached_steps time steps,
  *                     gb_plan_imaging_bytes(plan, cached_steps, with_rho,
  *                     imaging_format) bytes (may be NULL when
- *                     cached_steps == 0); those steps need no recompute in
+ *                     cached_steps == 0) on a 16-byte boundary (8-byte for
+ *                     bf16 and f24); those steps need no recompute in
  *                     the backward;
  *   with_rho          keep / compute the fields the density gradient needs;
  *   imaging_format    GB_IMG_F32, GB_IMG_F24 or GB_IMG_BF16.  The fields

@@ -99,3 +99,28 @@ def test_product_path_fails_loudly_without_gpu():
         acoustic_forward_kernel(nx=4, nz=4, dx=1.0, dz=1.0, nt=2, dt=1e-3, nabc=2, free_surface=False,
                                 src_x=[1], src_z=[1], src_n=1, src_v=torch.zeros(2), rcv_x=[1], rcv_z=[1], rcv_n=1,
                                 damp=torch.zeros(8, 8), vp=z, rho=z, device="cuda")
+
+
+@pytest.mark.parametrize("fmt,offset,ok", [(0, 0, True), (0, 8, False), (1, 8, True), (1, 4, False), (3, 8, True),
+                                           (3, 4, False)])
+def test_gradient_stores_start_where_the_kernels_can_access_them(lib, fmt, offset, ok):
+    """The kernels take an fp32 imaging buffer in 16-byte pieces and a bf16 or
+    fp24 one in 8-byte pieces, and so fp24 checkpoints: other starting
+    addresses are refused before anything is launched (a workspace of no
+    bytes ends the accepted calls there too)."""
+    from geobrain_b200 import _lib
+    d = _lib.ModelDesc(nz=40, nx=50, nabc=5, nt=10, n_shots=1, n_rcv=1, half=2, free_surface=0, dt=1e-3, dx=10.0)
+    one = np.ones(1, np.int64)
+    h = ctypes.c_void_p()
+    assert lib.gb_plan_create(ctypes.byref(d), *[one.ctypes.data] * 4, ctypes.byref(h)) == 0
+    try:
+        base = 1 << 20          # never dereferenced
+        for cached, ckpt in ((10, 0), (4, base), (4, base + offset)):
+            store = _lib.GradStore(ckpt or None, 3, _lib.CKPT_FORMATS["fp24"], base + offset, cached, 0, fmt)
+            want = _lib.GB_E_WORKSPACE if ok and ckpt % 8 == 0 else _lib.GB_E_ARG
+            args = [base] * 4
+            assert lib.gb_forward(h, *args, *[None] * 6, 0, None, ctypes.byref(store), base, 0, None) == want
+            assert lib.gb_backward(h, *args, base, None, None, ctypes.byref(store), base, None, None, base, 0,
+                                   None) == want
+    finally:
+        lib.gb_plan_destroy(h)
