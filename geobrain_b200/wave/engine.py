@@ -309,9 +309,8 @@ def unused_pool(device) -> int:
     the flat dictionary of all of them (180 us the two, 20 of which pay for
     pool_holds)."""
     stats = torch.cuda.memory_stats_as_nested_dict(device)
-    if not stats:                        # CUDA not initialised yet
-        return 0
-    return stats["reserved_bytes"]["all"]["current"] - stats["allocated_bytes"]["all"]["current"]
+    reserved, used = (stats.get(k, {}).get("all", {}).get("current", 0) for k in ("reserved_bytes", "allocated_bytes"))
+    return reserved - used
 
 
 def pool_holds(device, blocks: Sequence[int], other: int = 0) -> bool:
